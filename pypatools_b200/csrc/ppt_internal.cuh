@@ -177,7 +177,7 @@ __device__ __forceinline__ void ldg_f64x4(const double* p, double& a, double& b,
 __device__ __forceinline__ bool locate_axis(const AxisDev& a, double x, int& i, double& t) {
     if (!(x >= a.lo && x <= a.hi)) return false;   // NaN counts as outside
     if (a.uniform) {
-        double u = (x - a.lo) * a.inv_d;
+        double u = __dmul_rn(x - a.lo, a.inv_d);   // rounded before c is taken off, in every kernel
         int c = (int)floor(u);
         c = c < 0 ? 0 : (c > a.n - 2 ? a.n - 2 : c);
         double tt = u - (double)c;
@@ -221,18 +221,21 @@ __device__ __forceinline__ bool locate(const MapDev& m, V3 r, Cell& c) {
     return true;
 }
 
-// Reference lerp order (interpolators.py:127-135): x first, then y, then z.
+// Reference lerp order (interpolators.py:127-135): x first, then y, then z;
+// a u + b t with the fused product named, so that every kernel rounds alike.
+__device__ __forceinline__ double lerp_f64(double a, double b, double u, double t) {
+    return fma(a, u, __dmul_rn(b, t));
+}
+
 __device__ __forceinline__ double tri(double c000, double c100, double c010, double c110,
                                       double c001, double c101, double c011, double c111,
                                       double tx, double ty, double tz) {
-    double ux = 1.0 - tx, uy = 1.0 - ty, uz = 1.0 - tz;
-    double c00 = c000 * ux + c100 * tx;
-    double c01 = c001 * ux + c101 * tx;
-    double c10 = c010 * ux + c110 * tx;
-    double c11 = c011 * ux + c111 * tx;
-    double c0 = c00 * uy + c10 * ty;
-    double c1 = c01 * uy + c11 * ty;
-    return c0 * uz + c1 * tz;
+    const double ux = 1.0 - tx, uy = 1.0 - ty, uz = 1.0 - tz;
+    const double c00 = lerp_f64(c000, c100, ux, tx);
+    const double c01 = lerp_f64(c001, c101, ux, tx);
+    const double c10 = lerp_f64(c010, c110, ux, tx);
+    const double c11 = lerp_f64(c011, c111, ux, tx);
+    return lerp_f64(lerp_f64(c00, c10, uy, ty), lerp_f64(c01, c11, uy, ty), uz, tz);
 }
 
 // Gather the 8 corners of one field (record offset `off`) of a float64 map

@@ -262,6 +262,80 @@ __device__ __forceinline__ V3 half_kick(V3 w, V3 E, V3 B, double dt, double qm) 
     else return vay_u<EM, BM>(w, w_to_v<ALG>(w), E, B, dt, qm);
 }
 
+// The 8 corner records of one cell of a single-layout map, for the kernels
+// that keep them in registers from one field evaluation to the next
+// (keeps_corners below).  Corner q = di*4 + dj*2 + dk; the pad of a
+// four-element record is not kept.
+__host__ __device__ constexpr int layout_slots(int L) { return layout_width(L) == 4 ? 3 : layout_width(L); }
+
+template <int L>
+struct Corners {
+    int64_t base = -1;                 // node index of corner (0, 0, 0), -1: none
+    double v[8][layout_slots(L)];
+};
+template <>
+struct Corners<0> {};
+
+template <int L>
+__device__ __forceinline__ void load_corners(const MapDev& m, int64_t base, Corners<L>& K) {
+    constexpr int W = layout_width(L);
+    static_assert(W <= 4, "the six-component record is gathered field by field");
+    const double* p = static_cast<const double*>(m.data) + base * W;
+    const int64_t sx = m.sx * W, sy = m.sy * W;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const double* c = p + ((q >> 2) & 1) * sx + ((q >> 1) & 1) * sy + (q & 1) * W;
+        if constexpr (W == 4) {
+            double pad;
+            ldg_f64x4(c, K.v[q][0], K.v[q][1], K.v[q][2], pad);
+        } else if constexpr (W == 2) {
+            ldg_f64x2(c, K.v[q][0], K.v[q][1]);
+        } else {
+            K.v[q][0] = __ldg(c);
+        }
+    }
+    K.base = base;
+}
+
+// E and B from the kept corners: tri() per stored component.
+template <int L>
+__device__ __forceinline__ void interp_corners(const Corners<L>& K, const Cell& c, V3& E, V3& B) {
+    constexpr int S = layout_slots(L);
+    double o[S];
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+        o[k] = tri(K.v[0][k], K.v[4][k], K.v[2][k], K.v[6][k], K.v[1][k], K.v[5][k], K.v[3][k], K.v[7][k], c.tx, c.ty,
+                   c.tz);
+    if constexpr (L == kLayE) E = v3(o[0], o[1], o[2]);
+    else if constexpr (L == kLayB) B = v3(o[0], o[1], o[2]);
+    else if constexpr (L == kLayExEyBz) {
+        E = v3(o[0], o[1], 0.0);
+        B = v3(0.0, 0.0, o[2]);
+    } else if constexpr (L == kLayEzBz) {
+        E = v3(0.0, 0.0, o[0]);
+        B = v3(0.0, 0.0, o[1]);
+    } else {
+        B = v3(0.0, 0.0, o[0]);
+    }
+}
+
+// Which kernels keep the corner records between field evaluations.  RK4's
+// four evaluations of a step lie within one step's advance of each other (the
+// two middle ones almost coincide, and the last is next to the next step's
+// first), so most of its lanes find their cell unchanged and load nothing:
+// the L1 wavefronts of incoherent gathers are what bounds it.  The same holds
+// for Vay's one evaluation a step while a step is short against a cell.  The
+// Boris kernels are bound by issue, where a load that most lanes skip still
+// takes its slots, and run 6 blocks per SM on 80 registers: not there, nor for
+// the six-component record (96 registers).  Measured, kernel time: 1e6
+// electrons x 200 rk4_rel steps 15.3 -> 6.99 ms (L1 was at 80 %), 4e5 x 500
+// vay_rel steps 3.85 -> 2.87, vay 4.72 -> 2.73; protons of the ring, which change
+// their cell every step, 5e5 x 100 rk4_rel steps 1.46 -> 1.34, vay_rel 0.63 -> 0.60.
+__host__ __device__ constexpr bool keeps_corners(int alg, int L) {
+    return L != 0 && L != kLayFull &&
+           (alg == PPT_ALG_RK4 || alg == PPT_ALG_RK4_REL || alg == PPT_ALG_VAY || alg == PPT_ALG_VAY_REL);
+}
+
 struct Ctx {
     const FieldsDev* F;
     double dt, qm, omega, phase, t0;
@@ -292,8 +366,10 @@ __device__ __forceinline__ void build_rf_table64(double2* tab, int64_t step0, in
 // parts (E, B zero outside it); returns 1 when r is inside.  The cell search
 // is locate_axis's uniform branch, the interpolation tri() per stored
 // component, so the values are the run-time dispatch's (eval_fields_f64).
-template <int L>
-__device__ __forceinline__ int eval_single_f64(const MapDev& m, V3 r, V3& E, V3& B) {
+// (KEEP: K holds the cell of the last evaluation, and a point in the same
+// cell loads nothing.)
+template <int L, bool KEEP>
+__device__ __forceinline__ int eval_single_f64(const MapDev& m, V3 r, V3& E, V3& B, Corners<KEEP ? L : 0>& K) {
     E = v3(0.0, 0.0, 0.0);
     B = v3(0.0, 0.0, 0.0);
     if (!(axis_contains(m.ax[0], r.x) & axis_contains(m.ax[1], r.y) & axis_contains(m.ax[2], r.z))) return 0;
@@ -303,7 +379,7 @@ __device__ __forceinline__ int eval_single_f64(const MapDev& m, V3 r, V3& E, V3&
     const double x[3] = {r.x, r.y, r.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const double u = (x[a] - m.ax[a].lo) * m.ax[a].inv_d;
+        const double u = __dmul_rn(x[a] - m.ax[a].lo, m.ax[a].inv_d);
         ijk[a] = __double2int_rd(u);             // floor: u is in [0, n - 1] here
         tt[a] = u - (double)ijk[a];
     }
@@ -314,7 +390,7 @@ __device__ __forceinline__ int eval_single_f64(const MapDev& m, V3 r, V3& E, V3&
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const AxisDev& ax = m.ax[a];
-            const double u = (x[a] - ax.lo) * ax.inv_d;
+            const double u = __dmul_rn(x[a] - ax.lo, ax.inv_d);
             int cc = ijk[a];
             cc = cc < 0 ? 0 : (cc > ax.n - 2 ? ax.n - 2 : cc);
             const double t = u - (double)cc;
@@ -329,23 +405,13 @@ __device__ __forceinline__ int eval_single_f64(const MapDev& m, V3 r, V3& E, V3&
     if constexpr (L == kLayFull) {
         E = gather_f64s<8>(m, c, 0);
         B = gather_f64s<8>(m, c, 4);
-    } else if constexpr (L == kLayE) {
-        E = gather_f64s<4>(m, c, 0);
-    } else if constexpr (L == kLayB) {
-        B = gather_f64s<4>(m, c, 0);
-    } else if constexpr (L == kLayExEyBz) {
-        const V3 o = gather_f64s<4>(m, c, 0);
-        E = v3(o.x, o.y, 0.0);
-        B = v3(0.0, 0.0, o.z);
-    } else if constexpr (L == kLayEzBz) {
-        double o[2];
-        gather_slots_f64<2>(m, c, o);
-        E = v3(0.0, 0.0, o[0]);
-        B = v3(0.0, 0.0, o[1]);
+    } else if constexpr (KEEP) {
+        if (c.base != K.base) load_corners<L>(m, c.base, K);
+        interp_corners<L>(K, c, E, B);
     } else {
-        double o[1];
-        gather_slots_f64<1>(m, c, o);
-        B = v3(0.0, 0.0, o[0]);
+        Corners<L> now;
+        load_corners<L>(m, c.base, now);
+        interp_corners<L>(now, c, E, B);
     }
     return 1;
 }
@@ -359,11 +425,12 @@ __device__ __forceinline__ int eval_single_f64(const MapDev& m, V3 r, V3& E, V3&
 // per particle and b = g omega dt per step, (cos b, sin b) from the launch's
 // table or, beyond it, the same float64 expression, so a track's bits do not
 // depend on how it is split into launches; at RK4's stage times directly.
-template <bool RF, int L>
-__device__ __forceinline__ int fields_at(Ctx& c, V3 r, int64_t g, double toff, V3& E, V3& B) {
+template <bool RF, int L, bool KEEP = false>
+__device__ __forceinline__ int fields_at(Ctx& c, V3 r, int64_t g, double toff, V3& E, V3& B,
+                                         Corners<KEEP ? L : 0>& K) {
     int h;
     if constexpr (L == 0) h = eval_fields_f64(*c.F, r, E, B);
-    else h = eval_single_f64<L>(c.F->maps[0], r, E, B);
+    else h = eval_single_f64<L, KEEP>(c.F->maps[0], r, E, B, K);
     c.hits += h;
     if (RF) {
         constexpr int EM = L == 0 ? 7 : e_bits(L);
@@ -389,6 +456,12 @@ __device__ __forceinline__ int fields_at(Ctx& c, V3 r, int64_t g, double toff, V
         }
     }
     return h;
+}
+
+template <bool RF, int L>
+__device__ __forceinline__ int fields_at(Ctx& c, V3 r, int64_t g, double toff, V3& E, V3& B) {
+    Corners<0> none;
+    return fields_at<RF, L, false>(c, r, g, toff, E, B, none);
 }
 
 // Position advance of one step, r + v dt (pusher.py:395-404).
@@ -487,24 +560,26 @@ __device__ __forceinline__ int quiet_steps_f64(const FieldsDev& F, V3 r, V3 v, d
 // (vel: the velocity of the state w, kept between the steps of the u-state
 // algorithms, whose drift forms it anyway.)
 template <int ALG, bool RF, int L>
-__device__ __forceinline__ bool step(Ctx& c, V3& r, V3& w, V3& vel, int64_t g) {
+__device__ __forceinline__ bool step(Ctx& c, V3& r, V3& w, V3& vel, int64_t g,
+                                     Corners<keeps_corners(ALG, L) ? L : 0>& K) {
+    constexpr bool KEEP = keeps_corners(ALG, L);
     constexpr int EM = launch_e_bits(L), BM = launch_b_bits(L);
     const double dt = c.dt, qm = c.qm;
     if constexpr (ALG == PPT_ALG_RK4 || ALG == PPT_ALG_RK4_REL) {
         constexpr bool REL = ALG == PPT_ALG_RK4_REL;
         V3 E, B;
         const double h = 0.5 * dt;
-        fields_at<RF, L>(c, r, g, 0.0, E, B);
+        fields_at<RF, L, KEEP>(c, r, g, 0.0, E, B, K);
         V3 k1v = REL ? rk4_rel_deriv<EM, BM>(w, E, B, qm) : lorentz(w, E, B, qm);
         V3 k1r = w;
         V3 r2 = axpy(h, k1r, r), v2 = axpy(h, k1v, w);
-        fields_at<RF, L>(c, r2, g, h, E, B);
+        fields_at<RF, L, KEEP>(c, r2, g, h, E, B, K);
         V3 k2v = REL ? rk4_rel_deriv<EM, BM>(v2, E, B, qm) : lorentz(v2, E, B, qm);
         V3 r3 = axpy(h, v2, r), v3_ = axpy(h, k2v, w);
-        fields_at<RF, L>(c, r3, g, h, E, B);
+        fields_at<RF, L, KEEP>(c, r3, g, h, E, B, K);
         V3 k3v = REL ? rk4_rel_deriv<EM, BM>(v3_, E, B, qm) : lorentz(v3_, E, B, qm);
         V3 r4 = axpy(dt, v3_, r), v4 = axpy(dt, k3v, w);
-        fields_at<RF, L>(c, r4, g, dt, E, B);
+        fields_at<RF, L, KEEP>(c, r4, g, dt, E, B, K);
         V3 k4v = REL ? rk4_rel_deriv<EM, BM>(v4, E, B, qm) : lorentz(v4, E, B, qm);
         const double s6 = dt / 6.0;
         r = axpy(s6, axpy(2.0, v3_, axpy(2.0, v2, k1r)) + v4, r);
@@ -513,7 +588,7 @@ __device__ __forceinline__ bool step(Ctx& c, V3& r, V3& w, V3& vel, int64_t g) {
     } else if constexpr (ALG == PPT_ALG_YOSHIDA || ALG == PPT_ALG_YOSHIDA_REL) {
         constexpr bool REL = ALG == PPT_ALG_YOSHIDA_REL;
         V3 E, B;
-        fields_at<RF, L>(c, r, g, 0.0, E, B);
+        fields_at<RF, L, KEEP>(c, r, g, 0.0, E, B, K);
         const double cs[3] = {kYoC1, kYoC2, kYoC1};
         const double ds[3] = {kYoD1, kYoD2, kYoD1};
 #pragma unroll
@@ -528,7 +603,7 @@ __device__ __forceinline__ bool step(Ctx& c, V3& r, V3& w, V3& vel, int64_t g) {
         // With no map containing r and no constant field, E = B = 0 exactly and
         // the leapfrog, Boris and relativistic Boris updates return w unchanged
         // (every term they add is a signed zero), so they are skipped.
-        const bool any = fields_at<RF, L>(c, r, g, 0.0, E, B) != 0 || c.const_nz;
+        const bool any = fields_at<RF, L, KEEP>(c, r, g, 0.0, E, B, K) != 0 || c.const_nz;
         if constexpr (ALG == PPT_ALG_LEAPFROG) {
             if (any) w = axpy(dt, lorentz(w, E, B, qm), w);
             r = drift(r, w, dt);
@@ -620,6 +695,7 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
             }
         }
         V3 vel = w_to_v<ALG>(w);
+        Corners<keeps_corners(ALG, L) ? L : 0> K;
         // steps until the next record: record after global step g when (g+1) % rec == 0;
         // the records are numbered by counting on from the launch's first (with a 64-bit
         // division per record, one proton's 1000 recorded steps took 906 us, now 803)
@@ -640,7 +716,7 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
                 int i = 0;
                 while (i < seg) {
                     const V3 r0 = r;
-                    step<ALG, RF, L>(c, r, w, vel, g0 + i);
+                    step<ALG, RF, L>(c, r, w, vel, g0 + i, K);
                     ++i;
                     if (segment_hits_surface(P.surf, r0, r)) {
                         stopped = true;
@@ -671,13 +747,13 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
                         i += m;
                         quiet -= m;
                     } else {
-                        if (step<ALG, RF, L>(c, r, w, vel, g0 + i))
+                        if (step<ALG, RF, L>(c, r, w, vel, g0 + i, K))
                             quiet = quiet_steps_f64(P.F, r, state_velocity<ALG>(w, vel), P.dt);
                         ++i;
                     }
                 }
             } else {
-                for (int i = 0; i < seg; ++i) step<ALG, RF, L>(c, r, w, vel, g0 + i);
+                for (int i = 0; i < seg; ++i) step<ALG, RF, L>(c, r, w, vel, g0 + i, K);
             }
             k += seg;
             if ((int64_t)seg == to_rec) {
@@ -723,8 +799,16 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
 // of a pruned record layout fit 80 registers without spills (6 blocks: the
 // RF-gap map crossing 65.0 -> 62.9 ms against 96 registers and 5 blocks);
 // the run-time dispatch, the full record and the collision test would spill
-// there and keep 5.
+// there and keep 5.  The kernels that keep their corners: 4 blocks of RK4, 5 of
+// Vay (1e6 electrons x 200 rk4_rel steps, {Ex Ey Bz}: no bound 9.85 ms, 3 / 4 /
+// 5 blocks 7.70 / 6.99 / 8.03; 4e5 x 500 vay_rel steps 4 / 5 / 6 blocks 3.06 /
+// 2.87 / 3.56), one more for the one-element record (ring, 5e5 x 100 rk4_rel
+// steps 1.38 -> 1.34 ms, vay_rel 0.644 -> 0.600).
 __host__ __device__ constexpr int f64_min_blocks(int alg, bool coll, int layout) {
+    if (keeps_corners(alg, layout) && !coll) {
+        const int narrow = layout_width(layout) == 1 ? 1 : 0;
+        return ((alg == PPT_ALG_RK4 || alg == PPT_ALG_RK4_REL) ? 4 : 5) + narrow;
+    }
     return !alg_skips_free(alg) ? 1 : (!coll && layout != 0 && layout != kLayFull) ? 6 : 5;
 }
 
