@@ -419,6 +419,31 @@ int ppt_moments(int64_t n, const double* r, const double* v, double mass_mev,
 int ppt_moments_noalloc(int64_t n, const double* r, const double* v, double mass_mev,
                         double* out, void* stream);
 
+/* ---- host <-> device copies of pageable memory ---------------------------
+ * No reference counterpart (its arrays never leave the host).  A stager owns
+ * n_slots pinned buffers of slot_bytes on the current device and n_threads
+ * threads that copy between them and the caller's ordinary host memory; its
+ * copies run on copy_stream (a cudaStream_t of that device that only the
+ * stager uses; it must outlive the stager).  Calls may come from any thread. */
+typedef struct ppt_stager ppt_stager;   /* opaque */
+
+int ppt_stager_create(int64_t slot_bytes, int n_slots, int n_threads, void* copy_stream, ppt_stager** out);
+
+/* Host src -> device dst.  Returns once src has been read; work queued on
+ * `stream` after the call sees the copy, and the copy waits for what was queued
+ * on it before. */
+int ppt_stager_upload(ppt_stager* s, void* dst, const void* src, int64_t bytes, void* stream);
+
+/* Device src -> host dst, queued, once the cudaEvent_t `after` has happened
+ * (NULL: at once).  src must stay as it is, and dst is complete, when
+ * ppt_stager_finish returns. */
+int ppt_stager_download(ppt_stager* s, void* dst, const void* src, int64_t bytes, void* after);
+
+/* Wait for every download queued before the call. */
+int ppt_stager_finish(ppt_stager* s);
+
+int ppt_stager_destroy(ppt_stager* s);
+
 const char* ppt_last_error(void);
 int ppt_abi_version(void);
 

@@ -114,6 +114,11 @@ SIGNATURES = {
     "ppt_jobs_tick": (c_int, [c_void_p, c_int64, c_void_p]),
     "ppt_jobs_progress": (c_int, [c_void_p, POINTER(c_void_p), POINTER(c_void_p)]),
     "ppt_jobs_destroy": (c_int, [c_void_p]),
+    "ppt_stager_create": (c_int, [c_int64, c_int, c_int, c_void_p, POINTER(c_void_p)]),
+    "ppt_stager_upload": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
+    "ppt_stager_download": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
+    "ppt_stager_finish": (c_int, [c_void_p]),
+    "ppt_stager_destroy": (c_int, [c_void_p]),
     "ppt_last_error": (ctypes.c_char_p, []),
     "ppt_abi_version": (c_int, []),
 }

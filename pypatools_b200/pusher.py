@@ -443,7 +443,7 @@ HOST_POOL = HostResultPool(_pool_limit())
 
 
 def host_array(shape, dtype=np.float64):
-    """A numpy array for results the GPU fills, backed (from 64 MiB up) by an
+    """A numpy array for results the GPU fills, backed (from 4 MiB up) by an
     anonymous mapping advised for transparent huge pages, taken from
     ``HOST_POOL``: writing tens of GB into fresh 4 KiB pages is bound by page
     faults (27 GB/s measured with 24 threads on a B200 host), with huge pages
@@ -452,7 +452,7 @@ def host_array(shape, dtype=np.float64):
     it are gone."""
     import weakref
     nbytes = int(np.prod(shape)) * np.dtype(dtype).itemsize
-    if nbytes < (64 << 20) or not hasattr(mmap, "MADV_HUGEPAGE"):
+    if nbytes < (4 << 20) or not hasattr(mmap, "MADV_HUGEPAGE"):
         return np.empty(shape, dtype)
     m = HOST_POOL.take(nbytes)
     base = np.frombuffer(m, dtype=dtype)
@@ -463,37 +463,30 @@ def host_array(shape, dtype=np.float64):
 
 
 class HostStager:
-    """Host <-> device copies through a ring of pinned buffers.
-
-    Device -> numpy: each piece (``chunk`` bytes at most) goes device -> pinned
-    buffer on a copy stream (PCIe at ~50 GB/s on B200 hosts), then a worker
-    thread copies it into the destination numpy array (numpy releases the GIL
-    for the copy); the ring keeps ``slots`` pieces in flight.  The
-    destinations of ``track_batch`` are fresh huge-page-advised arrays
-    (``host_array``), whose first touch keeps up with the link; with 4 KiB
-    pages it ran at half of it.  Pinning the destination instead costs about a
-    second per 1.5 GB whenever the caller still holds earlier results, and a
-    device copy into pageable memory runs at ~2 GB/s.  numpy -> device
-    (``upload``): worker threads copy the pieces into the pinned buffers and
-    enqueue their host-to-device copies."""
+    """Host <-> device copies of ordinary numpy arrays through a ring of
+    pinned buffers (``ppt_stager_*``): native threads copy between the arrays
+    and the buffers, in pieces for all of them, while other pieces cross PCIe.
+    Pinning the arrays instead costs about a second per 1.5 GB, and a device
+    copy from or into pageable memory runs at 2-10 GB/s.  The destinations of
+    ``track_batch`` are recycled huge-page mappings (``host_array``), whose
+    first touch would otherwise be slower than the link."""
 
     _by_device = {}
 
-    def __init__(self, device, chunk=32 << 20, slots=24):
-        import threading
-        from concurrent.futures import ThreadPoolExecutor
+    def __init__(self, device, chunk=2 << 20, slots=96, threads=None):
+        import ctypes
+        import os
         torch = _torch()
         self.torch = torch
         self.device = device
-        self.chunk = int(chunk)
-        self.buffers = [torch.empty(self.chunk, dtype=torch.uint8, pin_memory=True) for _ in range(slots)]
-        self.views = [b.numpy() for b in self.buffers]
-        self.events = [torch.cuda.Event() for _ in range(slots)]
-        self.pending = [None] * slots
-        self.next = 0
+        self.lib = _lib.load()
+        if threads is None:
+            threads = max(1, min(12, (os.cpu_count() or 8) - 2))
         self.stream = torch.cuda.Stream(device=device)
-        self.pool = ThreadPoolExecutor(max_workers=slots)
-        self.lock = threading.Lock()
+        handle = ctypes.c_void_p()
+        with torch.cuda.device(device):
+            _lib.check(self.lib.ppt_stager_create(int(chunk), int(slots), int(threads), self.stream.cuda_stream, handle))
+        self.handle = handle.value
 
     @classmethod
     def for_device(cls, device):
@@ -509,69 +502,26 @@ class HostStager:
         contiguous numpy array ``dst`` (same bytes), after event ``after``.
         The caller keeps ``src`` alive (and unchanged) until ``finish()``
         returns: the copy stream reads it after this call returns."""
-        with self.lock:
-            self._copy(src, dst, after)
+        nbytes = src.numel() * src.element_size()
+        if nbytes != dst.nbytes or not src.is_contiguous() or not dst.flags.c_contiguous:
+            raise ValueError("src and dst must be contiguous and of the same size")
+        _lib.check(self.lib.ppt_stager_download(self.handle, dst.ctypes.data, src.data_ptr(), nbytes,
+                                                after.cuda_event if after is not None else None))
 
-    def _copy(self, src, dst, after):
-        torch = self.torch
-        sb = src.reshape(-1).view(torch.uint8)
-        db = dst.reshape(-1).view(np.uint8)
-        if after is not None:
-            self.stream.wait_event(after)
-        for a in range(0, db.size, self.chunk):
-            b = min(a + self.chunk, db.size)
-            k = self.next
-            self.next = (k + 1) % len(self.buffers)
-            if self.pending[k] is not None:
-                self.pending[k].result()          # the slot's previous piece is in its numpy array
-            with torch.cuda.stream(self.stream):
-                self.buffers[k][:b - a].copy_(sb[a:b], non_blocking=True)
-                self.events[k].record(self.stream)
-            self.pending[k] = self.pool.submit(self._land, k, db, a, b)
-
-    def _land(self, k, db, a, b):
-        self.events[k].synchronize()
-        np.copyto(db[a:b], self.views[k][:b - a])
-
-    def upload(self, src, dst):
+    def upload(self, src, dst, stream=None):
         """Copy the contiguous numpy array ``src`` into the contiguous device
-        tensor ``dst`` (same bytes) through the ring: worker threads copy the
-        pieces into the pinned buffers and enqueue each piece's host-to-device
-        copy on the copy stream.  Returns an event recorded after the last
-        piece; the caller's stream waits on it before reading ``dst``."""
-        torch = self.torch
-        sb = src.reshape(-1).view(np.uint8)
-        db = dst.reshape(-1).view(torch.uint8)
-        with self.lock:
-            staged = []
-            for a in range(0, sb.size, self.chunk):
-                b = min(a + self.chunk, sb.size)
-                k = self.next
-                self.next = (k + 1) % len(self.buffers)
-                if self.pending[k] is not None:
-                    self.pending[k].result()      # the slot's previous piece has landed or left
-                self.events[k].synchronize()      # and its last copy is done
-                self.pending[k] = self.pool.submit(self._stage, k, sb, db, a, b)
-                staged.append(self.pending[k])
-            for f in staged:
-                f.result()
-            ev = torch.cuda.Event()
-            ev.record(self.stream)
-        return ev
-
-    def _stage(self, k, sb, db, a, b):
-        torch = self.torch
-        np.copyto(self.views[k][:b - a], sb[a:b])
-        with torch.cuda.device(self.device), torch.cuda.stream(self.stream):
-            db[a:b].copy_(self.buffers[k][:b - a], non_blocking=True)
-            self.events[k].record(self.stream)
+        tensor ``dst`` (same bytes); ``src`` has been read when the call
+        returns, and work queued on ``stream`` (default: the current stream)
+        afterwards sees the copy."""
+        nbytes = dst.numel() * dst.element_size()
+        if nbytes != src.nbytes or not dst.is_contiguous() or not src.flags.c_contiguous:
+            raise ValueError("src and dst must be contiguous and of the same size")
+        st = stream if stream is not None else self.torch.cuda.current_stream(self.device)
+        _lib.check(self.lib.ppt_stager_upload(self.handle, dst.data_ptr(), src.ctypes.data, nbytes, st.cuda_stream))
 
     def finish(self):
-        with self.lock:
-            for k, f in enumerate(self.pending):
-                if f is not None:
-                    f.result()
-                    self.pending[k] = None
+        """Wait until every copy queued so far is in its numpy array."""
+        _lib.check(self.lib.ppt_stager_finish(self.handle))
 
 
 class PusherGPU:
@@ -654,12 +604,12 @@ class PusherGPU:
             raise ValueError(f"dt must be a scalar or have shape ({m},), got {d.shape}")
         return (float(d[0]) if m else 0.0), d
 
-    def _upload(self, a, device):
+    @staticmethod
+    def _upload(a, device):
         torch = _torch()
-        t = torch.from_numpy(a)
-        if device.type == "cuda":
-            t = t.pin_memory()
-        return t.to(device, non_blocking=True)
+        t = torch.empty(a.shape, dtype=torch.float64, device=device)
+        HostStager.for_device(device).upload(a, t)
+        return t
 
     # -- batch API -----------------------------------------------------------
     def push_batch(self, r_array, v_array, efield, bfield, dt):
@@ -716,21 +666,13 @@ class PusherGPU:
             return empty, empty.copy(), np.ones(0, dtype=bool)
         df = self._device_fields(efield, bfield)
         stager = HostStager.for_device(df.device)
-        uploads = []
-
-        def upload(a):
-            t = torch.empty(a.shape, dtype=torch.float64, device=df.device)
-            uploads.append(stager.upload(np.ascontiguousarray(a, dtype=np.float64), t))
-            return t
 
         rf_omega, rf_phase = 0.0, None
         if rf is not None:
             rf_omega = rf.omega
-            rf_phase = upload(np.broadcast_to(np.asarray(rf.phase, dtype=np.float64), (m,)))
-        d_r0, d_v0 = upload(r0), upload(v0)
-        with torch.cuda.device(df.device):
-            for ev in uploads:                 # the tracker reads them on this stream
-                torch.cuda.current_stream().wait_event(ev)
+            phase = np.broadcast_to(np.asarray(rf.phase, dtype=np.float64), (m,))
+            rf_phase = self._upload(np.ascontiguousarray(phase), df.device)
+        d_r0, d_v0 = self._upload(r0, df.device), self._upload(v0, df.device)
         surface = self.surface if _collide else None
         tr = DeviceTracker(self.algorithm, self.q_over_m, df, m, nsteps, dt, rec, self.precision,
                            rf_omega=rf_omega, rf_phase=rf_phase, t0=t0, record=True, device=self.device,
