@@ -515,7 +515,18 @@ __device__ __forceinline__ double drift_coord(double x, double v, double dt, int
     return x;
 }
 
+// A short run is quicker step by step: three independent FMAs a step, against
+// some hundred dependent instructions per coordinate (one proton, 1000 steps of
+// which 640 are field-free, kernel time with a record every 1 / 7 / 20 / 50
+// steps: 790 / 243 / 183 / 165 us closed form, 392 / 192 / 170 / 164 with runs of
+// up to 32 steps taken so).
+constexpr int kShortRun = 32;
+
 __device__ __forceinline__ V3 drift_run(V3 r, V3 v, double dt, int m) {
+    if (m <= kShortRun) {
+        for (; m > 0; --m) r = drift(r, v, dt);
+        return r;
+    }
     return v3(drift_coord(r.x, v.x, dt, m), drift_coord(r.y, v.y, dt, m), drift_coord(r.z, v.z, dt, m));
 }
 
@@ -640,8 +651,11 @@ __device__ __forceinline__ V3 state_velocity(V3 w, V3 vel) {
     else return w;
 }
 
-__device__ __forceinline__ void write_row(double* hist, int64_t rec, int64_t n, int64_t row, V3 a) {
-    double* p = hist + (rec * n + row) * 3;
+__device__ __forceinline__ double* row_at(double* hist, int64_t rec, int64_t n, int64_t row) {
+    return hist + (rec * n + row) * 3;
+}
+
+__device__ __forceinline__ void write_row(double* p, V3 a) {
     p[0] = a.x;
     p[1] = a.y;
     p[2] = a.z;
@@ -690,26 +704,33 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
                 w = half_kick<ALG, L>(w, E, B, -0.5 * P.dt, P.qm);
             }
             if (P.r_hist) {
-                write_row(P.r_hist, 0, n, row, r);
-                write_row(P.v_hist, 0, n, row, w_to_v<ALG>(w));
+                write_row(row_at(P.r_hist, 0, n, row), r);
+                write_row(row_at(P.v_hist, 0, n, row), w_to_v<ALG>(w));
             }
         }
         V3 vel = w_to_v<ALG>(w);
         Corners<keeps_corners(ALG, L) ? L : 0> K;
         // steps until the next record: record after global step g when (g+1) % rec == 0;
         // the records are numbered by counting on from the launch's first (with a 64-bit
-        // division per record, one proton's 1000 recorded steps took 906 us, now 803)
+        // division per record, one proton's 1000 recorded steps took 906 us, counting 803)
         const int nsteps = (int)P.nsteps;
         const int rec_every = P.rec_every > 0x7fffffff ? 0x7fffffff : (int)P.rec_every;
         const int64_t until64 = P.rec_every - 1 - (P.step0 % P.rec_every);
         int until = until64 > 0x7fffffff ? 0x7fffffff : (int)until64;   // beyond this launch anyway
         int64_t rec = P.step0 / P.rec_every + 1;
+        auto record = [&](V3 rr, V3 vv) {
+            if (P.r_hist) {
+                write_row(row_at(P.r_hist, rec, n, row), rr);
+                write_row(row_at(P.v_hist, rec, n, row), vv);
+            }
+            ++rec;
+        };
         // record-free segments: the inner loop carries only its counter
         int k = 0;
         int quiet = 0;   // upcoming steps known to be field-free (quiet_steps_f64)
         while (k < nsteps) {
-            const int64_t to_rec = (int64_t)until + 1;
-            const int seg = (int)(to_rec < (int64_t)(nsteps - k) ? to_rec : (int64_t)(nsteps - k));
+            const unsigned to_rec = (unsigned)until + 1u;
+            const int seg = (int)(to_rec < (unsigned)(nsteps - k) ? to_rec : (unsigned)(nsteps - k));
             const int64_t g0 = P.step0 + k;
             if constexpr (COLL) {
                 // one step at a time, each segment tested (no field-free runs)
@@ -725,12 +746,8 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
                 }
                 k += i;
                 // the reference records the step's position before its collision test
-                if ((int64_t)i == to_rec) {
-                    if (P.r_hist && rec < P.n_rec) {
-                        write_row(P.r_hist, rec, n, row, r);
-                        write_row(P.v_hist, rec, n, row, state_velocity<ALG>(w, vel));
-                    }
-                    ++rec;
+                if ((unsigned)i == to_rec) {
+                    record(r, state_velocity<ALG>(w, vel));
                     until = rec_every - 1;
                 } else {
                     until -= i;
@@ -756,12 +773,8 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
                 for (int i = 0; i < seg; ++i) step<ALG, RF, L>(c, r, w, vel, g0 + i, K);
             }
             k += seg;
-            if ((int64_t)seg == to_rec) {
-                if (P.r_hist && rec < P.n_rec) {
-                    write_row(P.r_hist, rec, n, row, r);
-                    write_row(P.v_hist, rec, n, row, state_velocity<ALG>(w, vel));
-                }
-                ++rec;
+            if ((unsigned)seg == to_rec) {
+                record(r, state_velocity<ALG>(w, vel));
                 until = rec_every - 1;
             } else {
                 until -= seg;
@@ -772,7 +785,7 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
                 V3 E, B;
                 fields_at<RF, L>(c, r, P.nsteps_total, 0.0, E, B);
                 w = half_kick<ALG, L>(w, E, B, 0.5 * P.dt, P.qm);
-                if (P.v_hist) write_row(P.v_hist, P.n_rec - 1, n, row, w_to_v<ALG>(w));
+                if (P.v_hist) write_row(row_at(P.v_hist, P.n_rec - 1, n, row), w_to_v<ALG>(w));
             }
         }
         st[s] = r.x;
@@ -795,7 +808,8 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
     return (unsigned)P.nsteps;
 }
 
-// Blocks of 128 per SM the launch bounds ask for: the Boris family's kernels
+// Blocks of 128 per SM the launch bounds ask for (small bunches, resident with
+// any of them, gain 1-8 % from no bound: not worth a second set of kernels): the Boris family's kernels
 // of a pruned record layout fit 80 registers without spills (6 blocks: the
 // RF-gap map crossing 65.0 -> 62.9 ms against 96 registers and 5 blocks);
 // the run-time dispatch, the full record and the collision test would spill
