@@ -52,10 +52,16 @@ class RFModulation:
         return 2.0 * math.pi * self.frequency
 
 
+_have_cuda = False
+
+
 def _torch():
+    global _have_cuda
     import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("PusherGPU needs a CUDA device (there is no CPU fallback)")
+    if not _have_cuda:      # asked once: the query costs 4 us, and a step asks five times
+        if not torch.cuda.is_available():
+            raise RuntimeError("PusherGPU needs a CUDA device (there is no CPU fallback)")
+        _have_cuda = True
     return torch
 
 
@@ -628,12 +634,15 @@ class PusherGPU:
         df = self._device_fields(efield, bfield)
         tr = DeviceTracker(self.algorithm, self.q_over_m, df, m, 1, dt, 1, self.precision, record=False,
                            stagger=False, device=self.device, dt_rows=dt_rows)
-        d_r, d_v = self._upload(r, df.device), self._upload(v, df.device)
+        # one copy each way
+        d_rv = self._upload(np.stack([r, v]), df.device)
         with torch.cuda.device(df.device):
-            tr.load(d_r, d_v)
-            tr.advance(1)
-            tr.store(d_r, d_v)
-        return d_r.cpu().numpy(), d_v.cpu().numpy()
+            stream = torch.cuda.current_stream()
+            tr.load(d_rv[0], d_rv[1], stream)
+            tr.advance(1, stream)
+            tr.store(d_rv[0], d_rv[1], stream)
+        rv = d_rv.cpu().numpy()
+        return rv[0], rv[1]
 
     def track_batch(self, r0_array, v0_array, efield, bfield, nsteps, dt, rec_every_n_steps=1, verbose=False,
                     *, rf=None, t0=0.0, _collide=True):
