@@ -361,15 +361,15 @@ __global__ void __launch_bounds__(kBlock) bi_scalars(int mode, const double* __r
 // registers: the vectors of up to twelve cells per thread stay resident, and
 // latency is covered by cells instead of warps.
 // B200, us per iteration, launched form -> this one: CG on 16^3 / 52 x 52 x 54 /
-// 64 x 64 x 128 cells 12.5 / 15.2 / 19.4 -> 4.3 / 5.3 / 8.2; BiCGSTAB 20.8 / 28.5 /
-// 39.5 -> 10.3 / 12.8 / 24.6, with a third of the iterations (bi_resident).
+// 64 x 64 x 128 cells 12.5 / 15.2 / 19.4 -> 4.3 / 5.6 / 8.4; BiCGSTAB 20.8 / 28.5 /
+// 39.5 -> 10.6 / 14.5 / 26.6, with a third of the iterations (bi_resident).
 // ---------------------------------------------------------------------------
 constexpr int kResThreads = 512;
 constexpr int kResWarps = kResThreads / 32;
 constexpr int kResMaxBlocks = 160;
 constexpr int kResMaxCg = 12;     // cells per thread: x, A r and A p in registers
 constexpr int kResMaxBi = 8;      // r, t, v and x in registers
-constexpr int kResMaxSums = 4;
+constexpr int kResMaxSums = 5;
 constexpr int kSpinLimit = 1 << 21;   // polls of one wait (~0.5 us each) before the solve gives up
 
 // A partial sum and the number of the wait it belongs to, written and read as
@@ -406,29 +406,30 @@ __device__ __forceinline__ unsigned long long poll(const Slot* p, double& v) {
 }
 
 struct GridSums {
-    double part[kResMaxSums][kResWarps];    // the block's warps
+    double part[8][kResWarps];              // the block's warps
     double all[kResMaxSums];                // the grid's sums
     int late;
 };
 
-// The warp's sums of N = 1, 2 or 4 values, value lane / (32 / N) in each lane:
-// while there are several, half the lanes pass one on and keep the other.
-template <int N>
-__device__ __forceinline__ double warp_sums(const double (&a)[N], int lane) {
-    double v = a[0];
-    if constexpr (N == 4) {
-        const bool up = lane & 16, odd = lane & 8;
-        double k0 = up ? a[2] : a[0], k1 = up ? a[3] : a[1];
-        k0 += __shfl_xor_sync(0xffffffffu, up ? a[0] : a[2], 16);
-        k1 += __shfl_xor_sync(0xffffffffu, up ? a[1] : a[3], 16);
-        v = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8);
-    } else if constexpr (N == 2) {
-        const bool up = lane & 16;
-        v = (up ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, up ? a[0] : a[1], 16);
-    }
+constexpr int sums_width(int n) { return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : 8; }
+
+// The warp's sums of W = 1, 2, 4 or 8 values, value lane / (32 / W) in each lane:
+// while there are several, half the lanes pass half of them on and keep the others.
+template <int W>
+__device__ __forceinline__ double warp_sums(const double (&a)[W], int lane, int o = 16) {
+    if constexpr (W == 1) {
+        double v = a[0];
 #pragma unroll
-    for (int o = 16 / N; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+        for (; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    } else {
+        const bool up = lane & o;
+        double half[W / 2];
+#pragma unroll
+        for (int i = 0; i < W / 2; ++i)
+            half[i] = (up ? a[i + W / 2] : a[i]) + __shfl_xor_sync(0xffffffffu, up ? a[i] : a[i + W / 2], o);
+        return warp_sums<W / 2>(half, lane, o >> 1);
+    }
 }
 
 // Wait number e of the grid: each of the N values summed over all threads of
@@ -442,9 +443,13 @@ __device__ __forceinline__ double warp_sums(const double (&a)[N], int lane) {
 // for four.
 template <int N>
 __device__ __forceinline__ bool grid_sums(Slot* slots, GridSums& G, unsigned long long e, double (&a)[N]) {
-    constexpr int L = 32 / N;                   // lanes of one value
+    constexpr int W = sums_width(N);
+    constexpr int L = 32 / W;                   // lanes of one value
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double v = warp_sums<N>(a, lane);
+    double wide[W];
+#pragma unroll
+    for (int n = 0; n < W; ++n) wide[n] = n < N ? a[n < N ? n : 0] : 0.0;
+    double v = warp_sums<W>(wide, lane);
     if (lane % L == 0) G.part[lane / L][warp] = v;
     __syncthreads();
     const int nb = (int)gridDim.x;
@@ -459,10 +464,10 @@ __device__ __forceinline__ bool grid_sums(Slot* slots, GridSums& G, unsigned lon
 #pragma unroll
         for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (nb == 1) {
-            if (j == 0) G.all[n] = v;
+            if (j == 0 && n < N) G.all[n] = v;
         } else {
             fence_gpu();          // the block's writes (ordered before this by the barrier) before its words
-            if (j == 0) publish(up + n * nb + blockIdx.x, v, e);
+            if (j == 0 && n < N) publish(up + n * nb + blockIdx.x, v, e);
         }
     }
     if (nb > 1) {
@@ -766,6 +771,8 @@ __device__ __forceinline__ double apply_row(const double* row, const double* x, 
     return apply_padded(row[0], w, x, at, sx, sy);
 }
 
+constexpr double kRhoRounding = 1e-28;     // (1e-14)^2, of |rhat|^2 |r|^2
+
 // BiCGSTAB over per-cell rows with the diagonal as right preconditioner (the
 // residual and the stopping test stay those of the rows as they are):
 // A is applied to p^ = p / d and s^ = s / d, d the cell's diagonal.  A row next
@@ -776,7 +783,9 @@ __device__ __forceinline__ double apply_row(const double* row, const double* x, 
 // 140; 36 x 59 x 117 to 1e-8: stopped at residuals between 4e-9 and 0.16, now 141
 // iterations).  p^ and s^ in padded bricks, x and rhat in shared memory, r (then
 // s), t, v and x in registers; p = d p^; of the padding cells r, v and d in lists.
-// rho = rhat.r = -omega rhat.t and r.r come from the sums taken with t.  A warp
+// rho = rhat.r and r.r come from the sums taken with t: r = s - omega t.  Once rho
+// is within the rounding of its sum, the iteration starts again from r as its
+// rhat; the launched form goes on, and stops unconverged where rho vanishes.  A warp
 // whose 32 cells all have the plain row takes its constants; another reads rows.
 template <int S>
 __global__ void __launch_bounds__(kResThreads, 1)
@@ -864,12 +873,15 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (!grid_sums(slots, G, epoch, first)) return;
     update_halo(P, t_pub, [&](int h, int, double rc) { halo_r[h] = rc; });
     double rr = first[0], rho = rr, beta = 0.0, omega = 1.0;
+    double rhat2 = rr;                 // |rhat|^2
+    bool fresh = true;                 // p = r: the first direction, and after a restart
+    bool restart = false;
     const double bb = first[1], tol2 = rel_tol * rel_tol * bb;
     int64_t it = 0;
     bool done = rr <= tol2 || rr == 0.0 || max_iter <= 0;
     // formed alike for a cell and for its copies in other bricks' padding
     auto direction = [&](double d, double ph, double vc, double rc) {
-        return it == 0 ? rc : fma(beta, fma(-omega, vc, d * ph), rc);
+        return fresh ? rc : fma(beta, fma(-omega, vc, d * ph), rc);
     };
     auto own_diag = [&](int s, double& d, double& inv) {
         d = A.diag;
@@ -890,6 +902,20 @@ __global__ void __launch_bounds__(kResThreads, 1)
         return apply_row(row[s] >= 0 ? rows[row[s]].w : coef + 7 * (int64_t)(-1 - row[s]), vec, at, P.sx, P.sy);
     };
     while (!done) {
+        if (restart) {
+            // rhat = r: the old one has nothing left to say about r
+            double sum[1] = {0.0};
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                rhat[threadIdx.x + s * kResThreads] = r[s];
+                sum[0] = fma(r[s], r[s], sum[0]);
+            }
+            if (!grid_sums(slots, G, ++epoch, sum)) return;
+            rr = rho = rhat2 = sum[0];
+            if (rr <= tol2 || rr == 0.0) break;
+            fresh = true;
+            restart = false;
+        }
         // p^ = (r + beta (p - omega v)) / d, v = A p^
         for (int h = threadIdx.x; h < P.halo; h += kResThreads) {
             const int at = P.dst[h];
@@ -903,6 +929,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             const double ph = inv * direction(d, p[at], v[s], r[s]);
             if (own[s] & kOwned) p[at] = ph;
         }
+        fresh = false;
         __syncthreads();
         double dv[1] = {0.0};
 #pragma unroll
@@ -913,7 +940,11 @@ __global__ void __launch_bounds__(kResThreads, 1)
             dv[0] = fma(rhat[l], v[s], dv[0]);           // rhat is zero past the brick's cells
         }
         if (!grid_sums(slots, G, ++epoch, dv)) return;
-        if (dv[0] == 0.0) break;                                 // breakdown
+        if (dv[0] == 0.0) {
+            restart = true;
+            done = ++it >= max_iter;
+            continue;
+        }
         const double alpha = rho / dv[0];
         // s = r - alpha v, t = A (s / d)
         update_halo(P, v_pub, [&](int h, int at, double vc) {
@@ -930,7 +961,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             if (own[s] & kOwned) half[own[s] & 0xffff] = inv * r[s];
         }
         __syncthreads();
-        double sum[4] = {0.0, 0.0, 0.0, 0.0};                    // t.s, t.t, rhat.t, s.s
+        double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0};               // t.s, t.t, rhat.s, rhat.t, s.s
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             const int l = threadIdx.x + s * kResThreads;
@@ -939,8 +970,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
             if (own[s] & kFace) t_pub[K.base + l] = tc;
             sum[0] = fma(r[s], t[s], sum[0]);
             sum[1] = fma(t[s], t[s], sum[1]);
-            sum[2] = fma(rhat[l], t[s], sum[2]);
-            sum[3] = fma(r[s], r[s], sum[3]);
+            sum[2] = fma(rhat[l], r[s], sum[2]);
+            sum[3] = fma(rhat[l], t[s], sum[3]);
+            sum[4] = fma(r[s], r[s], sum[4]);
         }
         if (!grid_sums(slots, G, ++epoch, sum)) return;
         omega = sum[1] > 0.0 ? sum[0] / sum[1] : 0.0;
@@ -953,12 +985,15 @@ __global__ void __launch_bounds__(kResThreads, 1)
             r[s] = fma(-omega, t[s], r[s]);
         }
         ++it;
-        rr = fma(omega, fma(omega, sum[1], -2.0 * sum[0]), sum[3]);
+        rr = fma(omega, fma(omega, sum[1], -2.0 * sum[0]), sum[4]);
         if (rr < 0.0) rr = 0.0;                                  // s = omega t to rounding
-        const double rho_new = -omega * sum[2];                  // rhat.s = rho - alpha rhat.v = 0
-        beta = (rho != 0.0 && omega != 0.0) ? (rho_new / rho) * (alpha / omega) : 0.0;
+        // (rhat.s vanishes but for rounding: without it rho would drift from rhat.r)
+        const double rho_new = fma(-omega, sum[3], sum[2]);
+        beta = omega != 0.0 ? (rho_new / rho) * (alpha / omega) : 0.0;
         rho = rho_new;
-        done = rr <= tol2 || rr == 0.0 || it >= max_iter || rho == 0.0 || omega == 0.0;
+        done = rr <= tol2 || rr == 0.0 || it >= max_iter;
+        // rhat.r is rounding alone (rhat lives on the cells with charge, r elsewhere by now)
+        restart = omega == 0.0 || rho * rho <= kRhoRounding * rhat2 * rr;
     }
 #pragma unroll
     for (int s = 0; s < S; ++s) {
