@@ -265,6 +265,12 @@ int ppt_surface_create(int64_t n_vertices, const double* vertices, int64_t n_tri
                        const int64_t* triangles, ppt_surface** out);
 int ppt_surface_destroy(ppt_surface* surface);
 
+/* Add a finer grid for the segment tests (ppt_track with a surface,
+ * ppt_surface_segments_hit) and what tells a track how far from the surface it
+ * is: the same hits, sooner.  Optional, once per surface,
+ * before it is used by other threads; synchronises. */
+int ppt_surface_refine(ppt_surface* surface);
+
 /* device bytes held, and the cell grid's dimensions */
 int ppt_surface_info(const ppt_surface* surface, int64_t* bytes, int32_t dims[3]);
 

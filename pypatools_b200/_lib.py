@@ -92,6 +92,7 @@ SIGNATURES = {
     "ppt_field_from_potential": (c_int, [POINTER(MeshDesc), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "ppt_surface_create": (c_int, [c_int64, c_void_p, c_int64, c_void_p, POINTER(c_void_p)]),
     "ppt_surface_destroy": (c_int, [c_void_p]),
+    "ppt_surface_refine": (c_int, [c_void_p]),
     "ppt_surface_info": (c_int, [c_void_p, POINTER(c_int64), POINTER(c_int32)]),
     "ppt_surface_axis_rays": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p]),
     "ppt_surface_segments_hit": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p]),

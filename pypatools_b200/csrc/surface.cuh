@@ -17,6 +17,9 @@
 // as the NumPy restatement's, bit for bit.
 #pragma once
 
+#include <mutex>
+#include <vector>
+
 #include "ppt_internal.cuh"
 
 namespace ppt {
@@ -30,6 +33,19 @@ struct SurfaceDev {
     int32_t dims[3];
     int32_t n_tri;
     const int32_t* trange;      // 6 per triangle: its first and last cell per axis (x0 x1 y0 y1 z0 z1)
+    // the grid the segment test uses: every cell cut into a few per axis
+    // (ppt_surface_refine; before it, the cells themselves)
+    const int32_t* seg_start;
+    const int32_t* seg_tri;
+    double seg_h[3];
+    double seg_inv_h[3];
+    int32_t seg_dims[3];
+    const double* plane;        // 4 per triangle: its plane's normal and offset (see beyond_plane)
+    double centre[3];           // the point the planes' offsets are from
+    double reach;               // the farthest the grid goes from it
+    const uint8_t* clearance;   // per cell: how many cells away (along any axis) the nearest listed triangle is,
+                                // at most 255 (NULL before ppt_surface_refine: no clear boxes)
+    double h[3];                // cell size
 };
 
 __device__ __forceinline__ double rn_dot(double ax, double ay, double az, double bx, double by, double bz) {
@@ -61,6 +77,22 @@ __device__ __forceinline__ bool segment_hits_triangle(const double* __restrict__
     return t >= 0.0 && t <= 1.0;
 }
 
+// Do both ends of a segment (a, b: from the planes' centre) lie on one side of
+// a triangle's plane, farther from it than the rounding of segment_hits_triangle
+// could bridge?  Then that test finds no hit.  With N = e1 x e2 it finds t as
+// N.(p0 - v0) / N.(p0 - p1), each rounded to within a few 2^-53 |e1| |e2| L, L the
+// lengths that enter; the planes are scaled by 1 / (|e1| |e2|), so a distance
+// above `margin` = 2^-43 L decides as the test would.  Four numbers and six FMAs
+// against nine and some fifty operations with a division: near a wall a step's
+// cell lists ten triangles, nearly all of them away from the segment.
+__device__ __forceinline__ bool beyond_plane(const double* __restrict__ plane, V3 a, V3 b, double margin) {
+    double nx, ny, nz, w;
+    ldg_f64x4(plane, nx, ny, nz, w);
+    const double sa = fma(nx, a.x, fma(ny, a.y, fma(nz, a.z, w)));
+    const double sb = fma(nx, b.x, fma(ny, b.y, fma(nz, b.z, w)));
+    return (sa > margin && sb > margin) || (sa < -margin && sb < -margin);
+}
+
 // Does the segment p0 -> p1 meet any triangle of the surface?  The cells of
 // the segment's bounding box are visited (one for the short steps of a
 // tracking run); a triangle listed in several of them may be tested twice.
@@ -69,22 +101,112 @@ __device__ __forceinline__ bool segment_hits_surface(const SurfaceDev& S, V3 p0,
     int lo[3], hi[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const double u0 = (fmin(a0[a], a1[a]) - S.lo[a]) * S.inv_h[a];
-        const double u1 = (fmax(a0[a], a1[a]) - S.lo[a]) * S.inv_h[a];
-        if (!(u1 >= 0.0 && u0 < (double)S.dims[a])) return false;   // beyond the mesh (or NaN)
+        const double u0 = (fmin(a0[a], a1[a]) - S.lo[a]) * S.seg_inv_h[a];
+        const double u1 = (fmax(a0[a], a1[a]) - S.lo[a]) * S.seg_inv_h[a];
+        if (!(u1 >= 0.0 && u0 < (double)S.seg_dims[a])) return false;   // beyond the mesh (or NaN)
         lo[a] = u0 <= 0.0 ? 0 : (int)u0;
-        hi[a] = u1 >= (double)(S.dims[a] - 1) ? S.dims[a] - 1 : (int)u1;
+        hi[a] = u1 >= (double)(S.seg_dims[a] - 1) ? S.seg_dims[a] - 1 : (int)u1;
     }
     const V3 d = v3(__dsub_rn(p1.x, p0.x), __dsub_rn(p1.y, p0.y), __dsub_rn(p1.z, p0.z));
+    const V3 centre = v3(S.centre[0], S.centre[1], S.centre[2]);
+    const V3 from = p0 - centre, to = p1 - centre;
+    const double margin = 0x1p-43 * (S.reach + fabs(from.x) + fabs(from.y) + fabs(from.z) + fabs(to.x) + fabs(to.y) +
+                                     fabs(to.z));
     for (int i = lo[0]; i <= hi[0]; ++i)
         for (int j = lo[1]; j <= hi[1]; ++j)
             for (int k = lo[2]; k <= hi[2]; ++k) {
-                const int cell = (i * S.dims[1] + j) * S.dims[2] + k;
-                const int end = S.cell_start[cell + 1];
-                for (int q = S.cell_start[cell]; q < end; ++q)
-                    if (segment_hits_triangle(S.tri + 9 * (int64_t)S.cell_tri[q], p0, d)) return true;
+                const int cell = (i * S.seg_dims[1] + j) * S.seg_dims[2] + k;
+                const int end = S.seg_start[cell + 1];
+                for (int q = S.seg_start[cell]; q < end; ++q) {
+                    const int64_t tri = S.seg_tri[q];
+                    if (beyond_plane(S.plane + 4 * tri, from, to, margin)) continue;
+                    if (segment_hits_triangle(S.tri + 9 * tri, p0, d)) return true;
+                }
             }
     return false;
+}
+
+// A box around a point in which no segment can meet the surface: the cells
+// closer than the nearest one that lists a triangle (clearance), or the part of
+// such a cell whose segment-grid cell lists none, or, beyond the
+// grid, everything beyond it on that side.  A tracked particle whose step ends
+// in the box it started in needs no test; it takes six comparisons where the
+// test takes some sixty instructions without a triangle in sight.  The box is
+// kept a millionth of a cell inside its cells, far more than the rounding of the
+// test's cell index, so a step it lets pass is one the test would have passed.
+struct ClearBox {
+    V3 lo, hi;
+};
+
+__device__ __forceinline__ ClearBox no_clear_box() {
+    return ClearBox{v3(INFINITY, INFINITY, INFINITY), v3(-INFINITY, -INFINITY, -INFINITY)};
+}
+
+__device__ __forceinline__ bool in_clear_box(const ClearBox& b, V3 p) {
+    return (p.x >= b.lo.x) & (p.x <= b.hi.x) & (p.y >= b.lo.y) & (p.y <= b.hi.y) & (p.z >= b.lo.z) & (p.z <= b.hi.z);
+}
+
+__device__ __forceinline__ ClearBox clear_box(const SurfaceDev& S, V3 p) {
+    if (S.clearance == nullptr) return no_clear_box();
+    const double pc[3] = {p.x, p.y, p.z};
+    double lo[3], hi[3];
+    int cell[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double u = (pc[a] - S.lo[a]) * S.inv_h[a];
+        if (!(u == u)) return no_clear_box();
+        cell[a] = u < 0.0 ? -1 : (u >= (double)S.dims[a] ? S.dims[a] : (int)u);
+        lo[a] = -INFINITY;
+        hi[a] = INFINITY;
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double m = 1e-6 * S.h[a];
+        if (cell[a] < 0) {
+            hi[a] = S.lo[a] - m;
+            return ClearBox{v3(lo[0], lo[1], lo[2]), v3(hi[0], hi[1], hi[2])};
+        }
+        if (cell[a] >= S.dims[a]) {
+            lo[a] = S.lo[a] + S.dims[a] * S.h[a] + m;
+            return ClearBox{v3(lo[0], lo[1], lo[2]), v3(hi[0], hi[1], hi[2])};
+        }
+    }
+    const int c = S.clearance[(cell[0] * S.dims[1] + cell[1]) * S.dims[2] + cell[2]];
+    if (c == 0) {
+        // next to the surface: the segment grid's cell, if that lists nothing
+        int s[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int at = (int)((pc[a] - S.lo[a]) * S.seg_inv_h[a]);
+            s[a] = at < S.seg_dims[a] ? at : S.seg_dims[a] - 1;
+            const double m = 1e-6 * S.seg_h[a];
+            lo[a] = S.lo[a] + s[a] * S.seg_h[a] + m;
+            hi[a] = S.lo[a] + (s[a] + 1) * S.seg_h[a] - m;
+        }
+        const int at = (s[0] * S.seg_dims[1] + s[1]) * S.seg_dims[2] + s[2];
+        if (S.seg_start[at + 1] > S.seg_start[at]) return no_clear_box();
+        return ClearBox{v3(lo[0], lo[1], lo[2]), v3(hi[0], hi[1], hi[2])};
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        // cells cell - (c - 1) .. cell + (c - 1) list nothing; nothing lies beyond the grid either
+        const double m = 1e-6 * S.h[a];
+        if (cell[a] - (c - 1) > 0) lo[a] = S.lo[a] + (cell[a] - (c - 1)) * S.h[a] + m;
+        if (cell[a] + c < S.dims[a]) hi[a] = S.lo[a] + (cell[a] + c) * S.h[a] - m;
+    }
+    return ClearBox{v3(lo[0], lo[1], lo[2]), v3(hi[0], hi[1], hi[2])};
+}
+
+// Steps of d (per step) a point in the box certainly stays in it.
+__device__ __forceinline__ int clear_steps(const ClearBox& b, V3 p, V3 d) {
+    const double x[3] = {p.x, p.y, p.z}, u[3] = {d.x, d.y, d.z};
+    const double lo[3] = {b.lo.x, b.lo.y, b.lo.z}, hi[3] = {b.hi.x, b.hi.y, b.hi.z};
+    double k = 1e9;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (u[a] != 0.0) k = fmin(k, u[a] > 0.0 ? (hi[a] - x[a]) / u[a] : (lo[a] - x[a]) / u[a]);
+    k = k * (1.0 - 1e-9) - 1.0;
+    return k >= 1.0 ? (int)k : 0;      // (NaN: 0)
 }
 
 // Ray p + t d (t >= 0) against one triangle: the hit's t, or -1.  The same
@@ -154,5 +276,9 @@ struct ppt_surface {
     int device;
     ppt::SurfaceDev dev;
     void* buf;          // one device allocation: triangles, cell offsets, cell lists
+    void* seg_buf;      // the segment grid's and the clearances', once refined
     size_t bytes;
+    std::vector<int32_t> start;  // the cells' list offsets
+    std::vector<double> boxes;   // the triangles' bounding boxes (lo x y z, hi x y z)
+    std::mutex refining;
 };

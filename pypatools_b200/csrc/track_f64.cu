@@ -3,34 +3,38 @@
 
 namespace ppt {
 
-template <int ALG, int L>
+// (L = 0, the run-time dispatch, has E whatever its maps store.)
+template <int ALG, bool COLL, int L>
 static void launch_layout(const TrackDev& P, bool rf, int grid, int block, cudaStream_t s) {
-    constexpr bool kE = layout_has_e(L);
+    constexpr bool kE = L == 0 || layout_has_e(L);
     const size_t smem = (size_t)P.rf_tab_n * sizeof(double2);
-    if (rf && kE) track_f64_kernel<ALG, kE, false, L><<<grid, block, smem, s>>>(P);
-    else track_f64_kernel<ALG, false, false, L><<<grid, block, 0, s>>>(P);
+    if (rf && kE) track_f64_kernel<ALG, kE, COLL, L><<<grid, block, smem, s>>>(P);
+    else track_f64_kernel<ALG, false, COLL, L><<<grid, block, 0, s>>>(P);
+}
+
+template <int ALG, bool COLL>
+static void launch_any(const TrackDev& P, bool rf, int grid, int block, cudaStream_t s) {
+    switch (f64_single_layout(P)) {
+        case kLayFull: launch_layout<ALG, COLL, kLayFull>(P, rf, grid, block, s); break;
+        case kLayE: launch_layout<ALG, COLL, kLayE>(P, rf, grid, block, s); break;
+        case kLayB: launch_layout<ALG, COLL, kLayB>(P, rf, grid, block, s); break;
+        case kLayExEyBz: launch_layout<ALG, COLL, kLayExEyBz>(P, rf, grid, block, s); break;
+        case kLayEzBz: launch_layout<ALG, COLL, kLayEzBz>(P, rf, grid, block, s); break;
+        case kLayBz: launch_layout<ALG, COLL, kLayBz>(P, rf, grid, block, s); break;
+        default: launch_layout<ALG, COLL, 0>(P, rf, grid, block, s);
+    }
 }
 
 template <int ALG>
 static cudaError_t launch_alg(const TrackDev& P, bool rf, bool coll, cudaStream_t s) {
     const int block = pick_block(P.n);
     const int grid = grid_for(P.n, block);
-    const size_t smem = (size_t)P.rf_tab_n * sizeof(double2);
     if (coll) {
-        if (rf) track_f64_kernel<ALG, true, true, 0><<<grid, block, smem, s>>>(P);
-        else track_f64_kernel<ALG, false, true, 0><<<grid, block, 0, s>>>(P);
-        return cudaGetLastError();
-    }
-    switch (f64_single_layout(P)) {
-        case kLayFull: launch_layout<ALG, kLayFull>(P, rf, grid, block, s); break;
-        case kLayE: launch_layout<ALG, kLayE>(P, rf, grid, block, s); break;
-        case kLayB: launch_layout<ALG, kLayB>(P, rf, grid, block, s); break;
-        case kLayExEyBz: launch_layout<ALG, kLayExEyBz>(P, rf, grid, block, s); break;
-        case kLayEzBz: launch_layout<ALG, kLayEzBz>(P, rf, grid, block, s); break;
-        case kLayBz: launch_layout<ALG, kLayBz>(P, rf, grid, block, s); break;
-        default:
-            if (rf) track_f64_kernel<ALG, true, false, 0><<<grid, block, smem, s>>>(P);
-            else track_f64_kernel<ALG, false, false, 0><<<grid, block, 0, s>>>(P);
+        // with a surface only Boris, the default pusher, has kernels for each record layout
+        if constexpr (ALG == PPT_ALG_BORIS) launch_any<ALG, true>(P, rf, grid, block, s);
+        else launch_layout<ALG, true, 0>(P, rf, grid, block, s);
+    } else {
+        launch_any<ALG, false>(P, rf, grid, block, s);
     }
     return cudaGetLastError();
 }

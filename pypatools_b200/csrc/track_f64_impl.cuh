@@ -668,6 +668,10 @@ __device__ __forceinline__ Ctx make_ctx(const TrackDev& P) {
 // All steps of one call for particle slot s (s < P.n); returns the steps done.
 // COLL: each step's segment is tested against the electrode surface after the
 // step's snapshot, and a particle that hits stops there (pusher.py:966-990).
+// Measured (kernel time, 1e6 protons x 1000 steps through a pipe and an aperture
+// plate, most of them stopped within 300): 15.1 ms with the test of every
+// triangle listed by a step's cells, 10.6 with the plane test in front of it and
+// clear boxes (surface.cuh), 7.2 on the refined segment grid.
 template <int ALG, bool RF, bool COLL, int L>
 __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_t s, Ctx& c) {
     {
@@ -728,20 +732,43 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
         // record-free segments: the inner loop carries only its counter
         int k = 0;
         int quiet = 0;   // upcoming steps known to be field-free (quiet_steps_f64)
+        ClearBox clear;
+        if constexpr (COLL) clear = no_clear_box();
         while (k < nsteps) {
             const unsigned to_rec = (unsigned)until + 1u;
             const int seg = (int)(to_rec < (unsigned)(nsteps - k) ? to_rec : (unsigned)(nsteps - k));
             const int64_t g0 = P.step0 + k;
             if constexpr (COLL) {
-                // one step at a time, each segment tested (no field-free runs)
+                // each segment is tested unless it ends in the clear box it starts in;
+                // a field-free run takes the steps that stay in it
                 int i = 0;
                 while (i < seg) {
+                    if constexpr (alg_skips_free(ALG)) {
+                        if (quiet > 0) {
+                            const V3 u = state_velocity<ALG>(w, vel);
+                            int m = clear_steps(clear, r, P.dt * u);
+                            m = min(m, min(quiet, seg - i));
+                            if (m > 0) {
+                                r = drift_run(r, u, P.dt, m);
+                                i += m;
+                                quiet -= m;
+                                continue;
+                            }
+                        }
+                    }
                     const V3 r0 = r;
-                    step<ALG, RF, L>(c, r, w, vel, g0 + i, K);
+                    const bool free = step<ALG, RF, L>(c, r, w, vel, g0 + i, K);
                     ++i;
-                    if (segment_hits_surface(P.surf, r0, r)) {
-                        stopped = true;
-                        break;
+                    if (!in_clear_box(clear, r)) {
+                        if (segment_hits_surface(P.surf, r0, r)) {
+                            stopped = true;
+                            break;
+                        }
+                        clear = clear_box(P.surf, r);
+                    }
+                    if constexpr (alg_skips_free(ALG)) {
+                        if (quiet > 0) --quiet;
+                        else if (free) quiet = quiet_steps_f64(P.F, r, state_velocity<ALG>(w, vel), P.dt);
                     }
                 }
                 k += i;
@@ -812,8 +839,9 @@ __device__ __forceinline__ unsigned track_f64_particle(const TrackDev& P, int64_
 // any of them, gain 1-8 % from no bound: not worth a second set of kernels): the Boris family's kernels
 // of a pruned record layout fit 80 registers without spills (6 blocks: the
 // RF-gap map crossing 65.0 -> 62.9 ms against 96 registers and 5 blocks);
-// the run-time dispatch, the full record and the collision test would spill
-// there and keep 5.  The kernels that keep their corners: 4 blocks of RK4, 5 of
+// the run-time dispatch and the full record would spill there and keep 5 (with
+// the collision test too: 8.3 / 7.5 / 7.2 ms with 4 / 5 / 6 blocks, 1e6 protons x
+// 1000 steps in a pipe).  The kernels that keep their corners: 4 blocks of RK4, 5 of
 // Vay (1e6 electrons x 200 rk4_rel steps, {Ex Ey Bz}: no bound 9.85 ms, 3 / 4 /
 // 5 blocks 7.70 / 6.99 / 8.03; 4e5 x 500 vay_rel steps 4 / 5 / 6 blocks 3.06 /
 // 2.87 / 3.56), one more for the one-element record (ring, 5e5 x 100 rk4_rel
@@ -823,7 +851,7 @@ __host__ __device__ constexpr int f64_min_blocks(int alg, bool coll, int layout)
         const int narrow = layout_width(layout) == 1 ? 1 : 0;
         return ((alg == PPT_ALG_RK4 || alg == PPT_ALG_RK4_REL) ? 4 : 5) + narrow;
     }
-    return !alg_skips_free(alg) ? 1 : (!coll && layout != 0 && layout != kLayFull) ? 6 : 5;
+    return !alg_skips_free(alg) ? 1 : (layout != 0 && layout != kLayFull) ? 6 : 5;
 }
 
 // L = 0: any fields; L = a kLay* mask: one uniform-grid map of that record

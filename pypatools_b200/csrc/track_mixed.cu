@@ -1196,20 +1196,49 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
             int k = 0;
             int quiet = 0;   // upcoming steps known to be field-free (quiet_steps)
             bool on_grid = false;   // the last steps were a field-free run (drift_steps)
+            ClearBox clear;
+            V3 at;
+            if constexpr (COLL) {
+                clear = no_clear_box();
+                at = mixed_position(P, cf, o);
+            }
             while (k < nsteps) {
                 const int64_t to_rec = (int64_t)until + 1;
                 const int seg = (int)(to_rec < (int64_t)(nsteps - k) ? to_rec : (int64_t)(nsteps - k));
                 const int64_t g0 = P.step0 + k;
                 if constexpr (COLL) {
-                    // one step at a time, each segment tested (no field-free runs)
+                    // each segment is tested unless it ends in the clear box it starts in;
+                    // a field-free run takes the steps that stay in it
                     int i = 0;
                     while (i < seg) {
-                        const V3 r0 = mixed_position(P, cf, o);
-                        family_step<ALG, RF, L>(c, cf, o, vh, vl, d, g0 + i);
+                        if (quiet > 0) {
+                            const V3 u = v3((double)vh[0] + (double)vl[0], (double)vh[1] + (double)vl[1],
+                                            (double)vh[2] + (double)vl[2]);
+                            int m = clear_steps(clear, at, P.dt * u);
+                            m = min(m, min(quiet, seg - i));
+                            if (m > 0) {
+                                float2 Q[3], U[3];
+                                drift_quanta(d, Q, U);
+                                drift_steps(cf, o, Q, U, g0 + i, m, on_grid);
+                                on_grid = true;
+                                at = mixed_position(P, cf, o);
+                                i += m;
+                                quiet -= m;
+                                continue;
+                            }
+                        }
+                        const V3 r0 = at;
+                        const int ahead = family_step<ALG, RF, L>(c, cf, o, vh, vl, d, g0 + i);
+                        quiet = quiet > 0 ? quiet - 1 : ahead;
+                        on_grid = false;
                         ++i;
-                        if (segment_hits_surface(C->surf, r0, mixed_position(P, cf, o))) {
-                            stopped = true;
-                            break;
+                        at = mixed_position(P, cf, o);
+                        if (!in_clear_box(clear, at)) {
+                            if (segment_hits_surface(C->surf, r0, at)) {
+                                stopped = true;
+                                break;
+                            }
+                            clear = clear_box(C->surf, at);
                         }
                     }
                     k += i;

@@ -55,8 +55,9 @@ class ElectrodeSurface:
         return ElectrodeSurface(np.concatenate([self.vertices, other.vertices]),
                                 np.concatenate([self.triangles, other.triangles + self.vertices.shape[0]]))
 
-    def handle(self, device):
-        """The device copy (created on first use on ``device``)."""
+    def handle(self, device, segments=False):
+        """The device copy (created on first use on ``device``); with
+        ``segments``, with the finer grid of the segment tests."""
         import torch
         dev = torch.device(device)
         idx = dev.index if dev.index is not None else torch.cuda.current_device()
@@ -69,6 +70,8 @@ class ElectrodeSurface:
                                                   self.triangles.shape[0], self.triangles.ctypes.data, out))
             h = out.value
             self._handles[idx] = h
+        if segments:
+            _lib.check(_lib.load().ppt_surface_refine(h))
         return h
 
     def info(self, device="cuda"):
@@ -90,7 +93,7 @@ class ElectrodeSurface:
         if m == 0:
             return {"hit_mask": np.zeros(0, dtype=bool)}
         dev = torch.device(device)
-        h = self.handle(dev)
+        h = self.handle(dev, segments=True)
         da, db = torch.from_numpy(a).to(dev), torch.from_numpy(b).to(dev)
         hit = torch.empty(m, dtype=torch.uint8, device=dev)
         with torch.cuda.device(da.device):

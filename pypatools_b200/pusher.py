@@ -147,7 +147,7 @@ class DeviceTracker:
             if precision != "fp64" and algorithm != "boris":
                 raise NotImplementedError("electrode surfaces run in the float64 form and in the mixed form's "
                                           "boris; use precision='fp64'")
-            self.surface = surface.handle(dev)
+            self.surface = surface.handle(dev, segments=True)
             self.active = torch.ones(n, dtype=torch.uint8, device=dev)
         if record:
             # stopped particles leave their later rows unwritten: NaN, as the
