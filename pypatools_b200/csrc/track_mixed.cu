@@ -116,6 +116,26 @@ __device__ __forceinline__ float2 tri8_pair_ff(const float2 q[8], float2 tx, flo
     return h;
 }
 
+// The 8 corner records of a cell, for the kernels that keep them in registers
+// from one field evaluation to the next (keeps_corners_f); corner q = di*4 + dj*2 + dk.
+template <int L>
+struct CornersF {
+    int64_t base = -1;                   // element offset of corner (0, 0, 0), -1: none
+    float v[8][layout_width(L)];
+};
+template <>
+struct CornersF<0> {};
+
+// RK4's four evaluations of a step lie within one step's advance of each other
+// (keeps_corners in track_f64_impl.cuh): with an incoherent bunch its gathers
+// are what bounds it.  1e6 electrons x 300 steps, {Ex Ey Bz}, kernel time: rk4_rel
+// 13.4 -> 9.0 ms, rk4 10.8 -> 7.4.  Not kept: one-element records, whose gathers
+// cost least (ring, rk4_rel: 2 % slower), and Vay and boris_rel, bound by issue
+// (electrons, vay: 11.8 -> 12.1 ms; RF gap, boris_rel: 5.6 -> 6.2).
+__host__ __device__ constexpr bool keeps_corners_f(int alg, int L) {
+    return (layout_width(L) == 2 || layout_width(L) == 4) && (alg == PPT_ALG_RK4 || alg == PPT_ALG_RK4_REL);
+}
+
 // Trilinear E/B at (cell, offset) from the float32 map of record layout L;
 // returns false when outside.  Components L does not store are compile-time
 // zeros, so the arithmetic that would multiply them vanishes from the
@@ -123,9 +143,9 @@ __device__ __forceinline__ float2 tri8_pair_ff(const float2 q[8], float2 tx, flo
 // (the host creates that layout whenever they are not zero).
 // El: the low parts of E's components (tri8_pair_ff).
 // fl: the offset's low words (zeros where only the high words are known).
-template <int L>
+template <int L, bool KEEP = false>
 __device__ __forceinline__ void gather_cell(const TrackMixDev& P, int i, int j, int k, float tx, float ty, float tz,
-                                            F3& E, F3& B, F3& El);
+                                            F3& E, F3& B, F3& El, CornersF<KEEP ? L : 0>& K);
 
 template <int L>
 __device__ __forceinline__ void field_init(const TrackMixDev& P, F3& E, F3& B, F3& El) {
@@ -139,24 +159,25 @@ __device__ __forceinline__ void field_init(const TrackMixDev& P, F3& E, F3& B, F
     }
 }
 
-template <int L>
+template <int L, bool KEEP>
 __device__ __forceinline__ bool gather_mixed(const TrackMixDev& P, const int cell[3], const float f[3],
-                                             const float fl[3], F3& E, F3& B, F3& El) {
+                                             const float fl[3], F3& E, F3& B, F3& El, CornersF<KEEP ? L : 0>& K) {
     field_init<L>(P, E, B, El);
     int i, j, k;
     float tx, ty, tz;
     if (!mixed_axis(cell[0], f[0], fl[0], P.G.n[0], i, tx)) return false;
     if (!mixed_axis(cell[1], f[1], fl[1], P.G.n[1], j, ty)) return false;
     if (!mixed_axis(cell[2], f[2], fl[2], P.G.n[2], k, tz)) return false;
-    gather_cell<L>(P, i, j, k, tx, ty, tz, E, B, El);
+    gather_cell<L, KEEP>(P, i, j, k, tx, ty, tz, E, B, El, K);
     return true;
 }
 
 // The trilinear fields of cell (i, j, k) at weights (tx, ty, tz), added to
 // the E, B field_init set.
-template <int L>
+// (KEEP: K holds the cell of the last evaluation; the same cell loads nothing.)
+template <int L, bool KEEP>
 __device__ __forceinline__ void gather_cell(const TrackMixDev& P, int i, int j, int k, float tx, float ty, float tz,
-                                            F3& E, F3& B, F3& El) {
+                                            F3& E, F3& B, F3& El, CornersF<KEEP ? L : 0>& K) {
     const MapDev& m = P.map;
     const float2 tx2 = make_float2(tx, tx), ty2 = make_float2(ty, ty), tz2 = make_float2(tz, tz);
     constexpr int W = layout_width(L);
@@ -180,6 +201,12 @@ __device__ __forceinline__ void gather_cell(const TrackMixDev& P, int i, int j, 
     }
     const float* p11 = p01 + (p10 - p00);
     const float* pc[4] = {p00, p01, p10, p11};
+    bool fetch = true;
+    if constexpr (KEEP) {
+        const int64_t base = p00 - static_cast<const float*>(m.data);
+        fetch = base != K.base;
+        K.base = base;
+    }
     // Components adjacent in the record are interpolated as packed pairs
     // (tri8_pair); a lone component takes tri8, the same operations.
     if constexpr (L == kLayFull) {
@@ -205,10 +232,24 @@ __device__ __forceinline__ void gather_cell(const TrackMixDev& P, int i, int j, 
     } else if constexpr (W == 4) {
         // three packed components and a pad: one 128-bit load per corner, two pairs
         float4 q[8];
+        if (fetch) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            q[2 * c] = __ldg(reinterpret_cast<const float4*>(pc[c]));
-            q[2 * c + 1] = __ldg(reinterpret_cast<const float4*>(pc[c] + 4));
+            for (int c = 0; c < 4; ++c) {
+                q[2 * c] = __ldg(reinterpret_cast<const float4*>(pc[c]));
+                q[2 * c + 1] = __ldg(reinterpret_cast<const float4*>(pc[c] + 4));
+            }
+            if constexpr (KEEP) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    K.v[c][0] = q[c].x;
+                    K.v[c][1] = q[c].y;
+                    K.v[c][2] = q[c].z;
+                }
+            }
+        }
+        if constexpr (KEEP) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) q[c] = make_float4(K.v[c][0], K.v[c][1], K.v[c][2], 0.0f);
         }
         float2 qa[8], qb[8];
 #pragma unroll
@@ -234,10 +275,23 @@ __device__ __forceinline__ void gather_cell(const TrackMixDev& P, int i, int j, 
     } else if constexpr (W == 2) {
         // kLayEzBz: one 64-bit load per corner, one pair
         float2 q[8];
+        if (fetch) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            q[2 * c] = __ldg(reinterpret_cast<const float2*>(pc[c]));
-            q[2 * c + 1] = __ldg(reinterpret_cast<const float2*>(pc[c] + 2));
+            for (int c = 0; c < 4; ++c) {
+                q[2 * c] = __ldg(reinterpret_cast<const float2*>(pc[c]));
+                q[2 * c + 1] = __ldg(reinterpret_cast<const float2*>(pc[c] + 2));
+            }
+            if constexpr (KEEP) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    K.v[c][0] = q[c].x;
+                    K.v[c][1] = q[c].y;
+                }
+            }
+        }
+        if constexpr (KEEP) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) q[c] = make_float2(K.v[c][0], K.v[c][1]);
         }
         float2 ol;
         const float2 o = tri8_pair_ff(q, tx2, ty2, tz2, ol);
@@ -247,10 +301,20 @@ __device__ __forceinline__ void gather_cell(const TrackMixDev& P, int i, int j, 
     } else {
         // kLayBz: one 32-bit load per corner
         float q[8];
+        if (fetch) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            q[2 * c] = __ldg(pc[c]);
-            q[2 * c + 1] = __ldg(pc[c] + 1);
+            for (int c = 0; c < 4; ++c) {
+                q[2 * c] = __ldg(pc[c]);
+                q[2 * c + 1] = __ldg(pc[c] + 1);
+            }
+            if constexpr (KEEP) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) K.v[c][0] = q[c];
+            }
+        }
+        if constexpr (KEEP) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) q[c] = K.v[c][0];
         }
         B = f3(0.0f, 0.0f, tri8([&](int c) { return q[c]; }, tx, ty, tz));
     }
@@ -277,10 +341,11 @@ __device__ __forceinline__ void mul_pair(double cf, float& eh, float& el) {
 template <bool RF, int L>
 __device__ __forceinline__ void rf_modulate(MixCtx& c, int64_t g, double toff, F3& E, F3& El);
 
-template <bool RF, int L>
+template <bool RF, int L, bool KEEP>
 __device__ __forceinline__ bool fields_mixed(MixCtx& c, const int cell[3], const float f[3], const float fl[3],
-                                             int64_t g, double toff, F3& E, F3& B, F3& El) {
-    bool in = gather_mixed<L>(*c.P, cell, f, fl, E, B, El);
+                                             int64_t g, double toff, F3& E, F3& B, F3& El,
+                                             CornersF<KEEP ? L : 0>& K) {
+    bool in = gather_mixed<L, KEEP>(*c.P, cell, f, fl, E, B, El, K);
     c.hits += in;
     rf_modulate<RF, L>(c, g, toff, E, El);
     return in || const_fields<L>(*c.P);
@@ -319,7 +384,15 @@ template <bool RF, int L>
 __device__ __forceinline__ bool fields_mixed(MixCtx& c, const int cell[3], const float f[3], const float fl[3],
                                              int64_t g, double toff, F3& E, F3& B) {
     F3 El;
-    return fields_mixed<RF, L>(c, cell, f, fl, g, toff, E, B, El);
+    CornersF<0> none;
+    return fields_mixed<RF, L, false>(c, cell, f, fl, g, toff, E, B, El, none);
+}
+
+template <bool RF, int L, bool KEEP>
+__device__ __forceinline__ bool fields_mixed(MixCtx& c, const int cell[3], const float f[3], const float fl[3],
+                                             int64_t g, double toff, F3& E, F3& B, CornersF<KEEP ? L : 0>& K) {
+    F3 El;
+    return fields_mixed<RF, L, KEEP>(c, cell, f, fl, g, toff, E, B, El, K);
 }
 
 
@@ -974,7 +1047,8 @@ __device__ __forceinline__ int quiet_steps(const TrackMixDev& P, const float cn[
 // field-free (0 when this step met a field or the particle may come back).
 template <int ALG, bool RF, int L>
 __device__ __forceinline__ int family_step(MixCtx& c, float cf[3], float2 o[3], float vh[3], float vl[3], Drift& d,
-                                           int64_t g) {
+                                           int64_t g, CornersF<keeps_corners_f(ALG, L) ? L : 0>& K) {
+    constexpr bool KEEP = keeps_corners_f(ALG, L);
     const TrackMixDev& P = *c.P;
     // (cf, hi) is normalised: hi in [0, 1] after steps that may see a field,
     // after field-free runs and steps (normalise), and in the loaded state
@@ -998,12 +1072,12 @@ __device__ __forceinline__ int family_step(MixCtx& c, float cf[3], float2 o[3], 
         bool have;
         if (ALG == PPT_ALG_BORIS && inner) {
             field_init<L>(P, E, B, El);
-            gather_cell<L>(P, cell[0], cell[1], cell[2], fn[0], fn[1], fn[2], E, B, El);
+            gather_cell<L, KEEP>(P, cell[0], cell[1], cell[2], fn[0], fn[1], fn[2], E, B, El, K);
             c.hits += 1u;
             rf_modulate<RF, L>(c, g, 0.0, E, El);
             have = true;
         } else {
-            have = fields_mixed<RF, L>(c, cell, fn, fln, g, 0.0, E, B, El);
+            have = fields_mixed<RF, L, KEEP>(c, cell, fn, fln, g, 0.0, E, B, El, K);
         }
         if (have) {
             F3 v = f3(vh[0], vh[1], vh[2]);
@@ -1051,12 +1125,13 @@ __device__ __forceinline__ int family_step(MixCtx& c, float cf[3], float2 o[3], 
 
 template <int ALG, bool RF, int L>
 __device__ __forceinline__ void mixed_step(MixCtx& c, int cell[3], float f[3], float fl[3], float vh[3], float vl[3],
-                                           Drift& d, int64_t g) {
+                                           Drift& d, int64_t g, CornersF<keeps_corners_f(ALG, L) ? L : 0>& K) {
+    constexpr bool KEEP = keeps_corners_f(ALG, L);
     const TrackMixDev& P = *c.P;
     F3 v = f3(vh[0], vh[1], vh[2]);
     if constexpr (ALG == PPT_ALG_VAY_REL) {
         F3 E, B;
-        fields_mixed<RF, L>(c, cell, f, fl, g, 0.0, E, B);
+        fields_mixed<RF, L, KEEP>(c, cell, f, fl, g, 0.0, E, B, K);
         F3 vn = vay_rel_f(v, E, B, P.qm, P.dtf);
         // increment relative to the float32 head keeps the low part's bits
         vel_add(vh, vl, vn - v);
@@ -1068,19 +1143,19 @@ __device__ __forceinline__ void mixed_step(MixCtx& c, int cell[3], float f[3], f
         int sc[3];
         float sf[3];
         const float sl[3] = {0.0f, 0.0f, 0.0f};   // stage positions: high words only
-        fields_mixed<RF, L>(c, cell, f, fl, g, 0.0, E, B);
+        fields_mixed<RF, L, KEEP>(c, cell, f, fl, g, 0.0, E, B, K);
         F3 k1 = REL ? rk4_rel_deriv_f(v, E, B, P.qm) : lorentz_f(v, E, B, P.qm);
         F3 v2 = v + h * k1;
         offset_point(P, cell, f, h * v, sc, sf);
-        fields_mixed<RF, L>(c, sc, sf, sl, g, 0.5 * P.dt, E, B);
+        fields_mixed<RF, L, KEEP>(c, sc, sf, sl, g, 0.5 * P.dt, E, B, K);
         F3 k2 = REL ? rk4_rel_deriv_f(v2, E, B, P.qm) : lorentz_f(v2, E, B, P.qm);
         F3 v3_ = v + h * k2;
         offset_point(P, cell, f, h * v2, sc, sf);
-        fields_mixed<RF, L>(c, sc, sf, sl, g, 0.5 * P.dt, E, B);
+        fields_mixed<RF, L, KEEP>(c, sc, sf, sl, g, 0.5 * P.dt, E, B, K);
         F3 k3 = REL ? rk4_rel_deriv_f(v3_, E, B, P.qm) : lorentz_f(v3_, E, B, P.qm);
         F3 v4 = v + dt * k3;
         offset_point(P, cell, f, dt * v3_, sc, sf);
-        fields_mixed<RF, L>(c, sc, sf, sl, g, P.dt, E, B);
+        fields_mixed<RF, L, KEEP>(c, sc, sf, sl, g, P.dt, E, B, K);
         F3 k4 = REL ? rk4_rel_deriv_f(v4, E, B, P.qm) : lorentz_f(v4, E, B, P.qm);
         // r_new - r = dt v + dt^2/6 (k1 + k2 + k3); v_new - v = dt/6 (k1 + 2k2 + 2k3 + k4)
         const float s6 = dt * (1.0f / 6.0f);
@@ -1182,6 +1257,7 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
             }
             if (P.r_hist) write_mixed_row(P, 0, row, cell, f, fl, vh, vl, true, alg_u_family(ALG));
         }
+        CornersF<keeps_corners_f(ALG, L) ? L : 0> K;
         Drift d;
         if constexpr (alg_u_family(ALG)) increment_u(P, vh, vl, d.dh, d.dl);
         else increment(P, vh, vl, d.dh, d.dl);
@@ -1228,7 +1304,7 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
                             }
                         }
                         const V3 r0 = at;
-                        const int ahead = family_step<ALG, RF, L>(c, cf, o, vh, vl, d, g0 + i);
+                        const int ahead = family_step<ALG, RF, L>(c, cf, o, vh, vl, d, g0 + i, K);
                         quiet = quiet > 0 ? quiet - 1 : ahead;
                         on_grid = false;
                         ++i;
@@ -1268,7 +1344,7 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
                         i += m;
                         quiet -= m;
                     } else {
-                        quiet = family_step<ALG, RF, L>(c, cf, o, vh, vl, d, g0 + i);
+                        quiet = family_step<ALG, RF, L>(c, cf, o, vh, vl, d, g0 + i, K);
                         on_grid = false;
                         ++i;
                     }
@@ -1293,7 +1369,7 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
             }
         } else {
             for (int k = 0; k < nsteps; ++k) {
-                mixed_step<ALG, RF, L>(c, cell, f, fl, vh, vl, d, P.step0 + k);
+                mixed_step<ALG, RF, L>(c, cell, f, fl, vh, vl, d, P.step0 + k, K);
                 if (until == 0) {
                     const int64_t rec = (P.step0 + k + 1) / P.rec_every;
                     if (P.r_hist && rec < P.n_rec) write_mixed_row(P, rec, row, cell, f, fl, vh, vl, true);
@@ -1355,8 +1431,21 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
     }
 }
 
-template <int ALG, bool RF, int L>
-__global__ void __launch_bounds__(128) track_mixed_kernel(const __grid_constant__ TrackMixDev P) {
+// Blocks of 128 per SM asked for (0: no bound) by the kernels that keep their
+// corners: 6 with four-element records, 7 with two (1e6 electrons x 300 rk4_rel
+// steps with 6 / 7 / 8: 8.97 / 9.03 / 9.43 ms; RF gap, 1e6 x 200 rk4 steps 6.25 /
+// 6.03 / 6.09, 6.08 without kept corners).  WIDE: a bunch that three blocks per SM
+// hold is as resident with all the registers it can use, and its latency gains by
+// them (4096 protons x 1000 rk4 steps: 1.20 ms without kept corners, 1.28 with a
+// bound of 6, 1.04 without a bound).
+constexpr int64_t kWideParticles = 148 * 3 * 128;
+
+__host__ __device__ constexpr int mixed_min_blocks(int alg, int L, bool wide) {
+    return !keeps_corners_f(alg, L) ? 0 : wide ? 3 : layout_width(L) == 4 ? 6 : 7;
+}
+
+template <int ALG, bool RF, int L, bool WIDE = false>
+__global__ void __launch_bounds__(128, mixed_min_blocks(ALG, L, WIDE)) track_mixed_kernel(const __grid_constant__ TrackMixDev P) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     unsigned steps_done = 0;
     MixCtx c{&P, 0.0, 0u, 0.0, 0.0, nullptr, 0};
@@ -1453,8 +1542,15 @@ static cudaError_t launch_mixed_layout(const TrackMixDev* P, const JobQueueDev* 
         const int block = pick_block(P->n);
         const int g = grid_for(P->n, block);
         const size_t smem = (size_t)P->rf_tab_n * sizeof(double2);
-        if (rf && kE) track_mixed_kernel<ALG, kE, L><<<g, block, smem, s>>>(*P);
-        else track_mixed_kernel<ALG, false, L><<<g, block, 0, s>>>(*P);
+        constexpr bool kWide = keeps_corners_f(ALG, L);
+        if (kWide && P->n <= kWideParticles) {
+            if (rf && kE) track_mixed_kernel<ALG, kE, L, kWide><<<g, block, smem, s>>>(*P);
+            else track_mixed_kernel<ALG, false, L, kWide><<<g, block, 0, s>>>(*P);
+        } else if (rf && kE) {
+            track_mixed_kernel<ALG, kE, L><<<g, block, smem, s>>>(*P);
+        } else {
+            track_mixed_kernel<ALG, false, L><<<g, block, 0, s>>>(*P);
+        }
     } else {
         const size_t smem = Q->chunk + 1 <= kRfTable ? (size_t)(Q->chunk + 1) * sizeof(double2) : 0;
         if (rf && kE) track_mixed_jobs_kernel<ALG, kE, L><<<grid, kJobBlock, smem, s>>>(*Q);
