@@ -363,9 +363,8 @@ class DeviceTracker:
         _lib.check(self.lib.ppt_cell_sort(self.state, self.dfields.fields, self.order.data_ptr(),
                                           self.rf_phase.data_ptr() if self.rf_phase is not None else None,
                                           scratch.data_ptr(), self._stream(stream)))
-        # keys, tile scan, top scan, scan add, scatter, then one copy-back per
-        # permuted array (state block(s), order, RF phase)
-        self.launches += 5 + (1 if self.precision == "fp64" else 2) + 1 + (1 if self.rf_phase is not None else 0)
+        # keys, tile scan, top scan, scan add, scatter, unpack
+        self.launches += 6
 
     def store(self, r, v, stream=None):
         """Write the current state as (n,3) float64 r, v in row order."""
