@@ -179,30 +179,15 @@ __global__ void scan_add(int64_t nb, uint32_t* __restrict__ offset, const uint32
 template <bool F64>
 struct Record {
     static constexpr int kWords = F64 ? 16 : 20;
-    static constexpr int kColumns = F64 ? 12 : 15;   // state words
     static constexpr int kOrder = F64 ? 12 : 16;     // first word of the row, then of the phase
 };
 
+// Slot s's record to position d.
 template <bool F64>
-__global__ void __launch_bounds__(256) sort_scatter(int64_t n, const uint32_t* __restrict__ key,
-                                                    uint32_t* __restrict__ offset, const uint32_t* __restrict__ ctrl,
-                                                    const uint32_t* __restrict__ src_a,
-                                                    const uint32_t* __restrict__ src_b,
-                                                    const uint2* __restrict__ order, const uint2* __restrict__ phase,
-                                                    uint4* __restrict__ records) {
+__device__ __forceinline__ void write_record(int64_t n, int64_t s, int64_t d, const uint32_t* __restrict__ src_a,
+                                             const uint32_t* __restrict__ src_b, const uint2* __restrict__ order,
+                                             const uint2* __restrict__ phase, uint4* __restrict__ records) {
     using R = Record<F64>;
-    if (!sort_wanted(ctrl, n)) return;
-    int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const uint32_t b = key[s];
-    const unsigned active = __activemask();
-    const unsigned same = __match_any_sync(active, b);
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(same) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(offset + b, (uint32_t)__popc(same));
-    base = __shfl_sync(same, base, leader);
-    const int64_t d = (int64_t)base + __popc(same & ((1u << lane) - 1u));
     uint32_t w[R::kWords];
     if constexpr (F64) {
         const uint2* col = reinterpret_cast<const uint2*>(src_a);
@@ -230,8 +215,49 @@ __global__ void __launch_bounds__(256) sort_scatter(int64_t n, const uint32_t* _
     for (int q = 0; q < R::kWords / 4; ++q) out[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
 }
 
-// The sorted records back into the columns (only when the sort ran), 128 at a
-// time through shared memory (an odd stride: no bank conflicts).
+template <bool F64>
+__global__ void __launch_bounds__(256) sort_scatter(int64_t n, const uint32_t* __restrict__ key,
+                                                    uint32_t* __restrict__ offset, const uint32_t* __restrict__ ctrl,
+                                                    const uint32_t* __restrict__ src_a,
+                                                    const uint32_t* __restrict__ src_b,
+                                                    const uint2* __restrict__ order, const uint2* __restrict__ phase,
+                                                    uint4* __restrict__ records) {
+    if (!sort_wanted(ctrl, n)) return;
+    int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const uint32_t b = key[s];
+    const unsigned active = __activemask();
+    const unsigned same = __match_any_sync(active, b);
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(same) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(offset + b, (uint32_t)__popc(same));
+    base = __shfl_sync(same, base, leader);
+    const int64_t d = (int64_t)base + __popc(same & ((1u << lane) - 1u));
+    write_record<F64>(n, s, d, src_a, src_b, order, phase, records);
+}
+
+// Back to row order: slot s to position order[s].  (order is a permutation of
+// 0 .. n-1, kept so by the sorts; a slot with a value outside is skipped.)
+// A gather of the columns through the inverse permutation read a 32-byte sector
+// for every word of every slot and needed the columns copied back.  B200, gather ->
+// records, the random order of a fresh sort: 1e7 mixed slots 3.12 -> 1.35 ms, 1e6
+// 0.117 -> 0.101, 20 000 30 -> 13 us, 1e7 float64 1.37 -> 0.87; a 6000-step track
+// of 6e6 mixed protons (8 sorts and one return) 4.04 -> 3.47 in all.
+template <bool F64>
+__global__ void __launch_bounds__(256) restore_scatter(int64_t n, const uint32_t* __restrict__ src_a,
+                                                       const uint32_t* __restrict__ src_b,
+                                                       const uint2* __restrict__ order,
+                                                       const uint2* __restrict__ phase,
+                                                       uint4* __restrict__ records) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const int64_t d = reinterpret_cast<const int64_t*>(order)[s];
+    if (d >= 0 && d < n) write_record<F64>(n, s, d, src_a, src_b, order, phase, records);
+}
+
+// The permuted records back into the columns (after a sort, ctrl given, only when
+// it ran), 128 at a time through shared memory (an odd stride: no bank conflicts).
 constexpr int kUnpack = 128;
 
 template <bool F64>
@@ -240,7 +266,7 @@ __global__ void __launch_bounds__(kUnpack) sort_unpack(int64_t n, const uint32_t
                                                        uint32_t* __restrict__ dst_b, uint2* __restrict__ order,
                                                        uint2* __restrict__ phase) {
     using R = Record<F64>;
-    if (!sort_wanted(ctrl, n)) return;
+    if (ctrl && !sort_wanted(ctrl, n)) return;
     __shared__ uint32_t tile[kUnpack * (R::kWords + 1)];
     const int64_t first = blockIdx.x * (int64_t)kUnpack;
     const int here = (int)(n - first < kUnpack ? n - first : kUnpack);
@@ -262,54 +288,16 @@ __global__ void __launch_bounds__(kUnpack) sort_unpack(int64_t n, const uint32_t
 #pragma unroll
         for (int c = 0; c < 12; ++c) dst_b[c * n + s] = w[3 + c];
     }
-    order[s] = make_uint2(w[R::kOrder], w[R::kOrder + 1]);
+    // back in row order (no ctrl) every slot is its own row
+    order[s] = ctrl ? make_uint2(w[R::kOrder], w[R::kOrder + 1])
+                    : make_uint2((uint32_t)s, (uint32_t)((uint64_t)s >> 32));
     if (phase) phase[s] = make_uint2(w[R::kOrder + 2], w[R::kOrder + 3]);
-}
-
-// Back to row order: position d takes the slot s with order[s] = d.  First
-// the inverse, perm[order[s]] = s (order is a permutation of 0 .. n-1, kept
-// so by the sorts; a value outside [0, n) is skipped), then a gather that
-// reads the slots scattered and writes every column in order: for the cell
-// order of a bunch that has crossed its map, 2.8 ms against 6.8 ms for the
-// scatter (slot s written to position order[s]) at 1e7 mixed-form particles.
-// (The cell sort keeps its scatter: for the random order of a fresh bunch the
-// gather took 4.5 ms against 2.4 ms.)
-__global__ void restore_inverse(int64_t n, const int64_t* __restrict__ order, uint32_t* __restrict__ perm) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const int64_t d = order[s];
-    if (d >= 0 && d < n) perm[d] = (uint32_t)s;
-}
-
-// Position d of the permuted copy takes slot perm[d]: ncols64 columns of
-// 8-byte words and na + nb columns of 4-byte words from two sources (mixed
-// state: the int32 cells, then the float32 columns) into one destination
-// block, and the RF phase.  perm values outside [0, n) (positions no slot
-// claimed; none for a permutation) leave position d unwritten.
-__global__ void restore_gather(int64_t n, const uint32_t* __restrict__ perm, int ncols64,
-                               const double* __restrict__ src64, double* __restrict__ dst64, int na,
-                               const uint32_t* __restrict__ src_a, int nb, const uint32_t* __restrict__ src_b,
-                               uint32_t* __restrict__ dst32, const double* __restrict__ phase,
-                               double* __restrict__ phase_out) {
-    const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (d >= n) return;
-    const uint32_t s = perm[d];
-    if ((int64_t)s >= n) return;
-    for (int c = 0; c < ncols64; ++c) dst64[c * n + d] = src64[c * n + s];
-    for (int c = 0; c < na; ++c) dst32[c * n + d] = src_a[c * n + s];
-    for (int c = 0; c < nb; ++c) dst32[(na + c) * n + d] = src_b[c * n + s];
-    if (phase) phase_out[d] = phase[s];
-}
-
-__global__ void iota_rows(int64_t n, int64_t* __restrict__ order) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s < n) order[s] = s;
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct SortLayout {
-    size_t key, count, tiles, ctrl, tmp64, tmp32, order, phase, perm, total;
+    size_t key, count, tiles, ctrl, records, total;
 };
 
 static SortLayout sort_layout(int64_t n) {
@@ -320,27 +308,29 @@ static SortLayout sort_layout(int64_t n) {
     L.count = o; o += align256(nb * 4);
     L.tiles = o; o += align256((nb / kScanTile + 2) * 4);
     L.ctrl = o;  o += 256;
-    L.tmp64 = o; o += align256((size_t)n * 6 * 8);     // float64 state
-    L.tmp32 = o; o += align256((size_t)n * 15 * 4);    // mixed: 3 int32 + 12 float32 columns
-    L.order = o; o += align256((size_t)n * 8);
-    L.phase = o; o += align256((size_t)n * 8);
-    L.perm = o;  o += align256((size_t)n * 4);    // restore: the inverse of order
+    L.records = o; o += align256((size_t)n * Record<false>::kWords * 4 + 16);   // 16: see records_in
     L.total = o;
     return L;
 }
 
+// the records' place in a scratch buffer, on a 16-byte boundary whatever that is on
+static uint4* records_in(char* scratch, const SortLayout& L) {
+    return reinterpret_cast<uint4*>((reinterpret_cast<uintptr_t>(scratch + L.records) + 15) & ~(uintptr_t)15);
+}
+
+// slots -> records -> columns: a sort's permutation, or (key NULL) back to row order
 template <bool F64>
 static void permute(const ppt_state* st, const uint32_t* key, uint32_t* offset, const uint32_t* ctrl, int64_t* order,
-                    double* rf_phase, void* records, cudaStream_t s) {
+                    double* rf_phase, uint4* records, cudaStream_t s) {
     const int64_t n = st->n;
     uint32_t* a = F64 ? reinterpret_cast<uint32_t*>(st->f64) : reinterpret_cast<uint32_t*>(st->i32);
     uint32_t* b = reinterpret_cast<uint32_t*>(st->f32);
     uint2* row = reinterpret_cast<uint2*>(order);
     uint2* phase = reinterpret_cast<uint2*>(rf_phase);
-    sort_scatter<F64><<<grid_for(n, 256), 256, 0, s>>>(n, key, offset, ctrl, a, b, row, phase,
-                                                       static_cast<uint4*>(records));
-    sort_unpack<F64><<<grid_for(n, kUnpack), kUnpack, 0, s>>>(n, static_cast<const uint32_t*>(records), ctrl, a, b, row,
-                                                              phase);
+    if (key) sort_scatter<F64><<<grid_for(n, 256), 256, 0, s>>>(n, key, offset, ctrl, a, b, row, phase, records);
+    else restore_scatter<F64><<<grid_for(n, 256), 256, 0, s>>>(n, a, b, row, phase, records);
+    sort_unpack<F64><<<grid_for(n, kUnpack), kUnpack, 0, s>>>(n, reinterpret_cast<const uint32_t*>(records), ctrl, a, b,
+                                                              row, phase);
 }
 
 }  // namespace ppt
@@ -398,9 +388,7 @@ extern "C" int ppt_cell_sort(ppt_state* st, const ppt_fields* fields, int64_t* o
     scan_tiles<<<ntiles, kScanTile, 0, s>>>(nb, count, count, tiles, ctrl, n);
     scan_top<<<1, kScanTile, 0, s>>>(ntiles, tiles, ctrl, n);
     scan_add<<<grid_for(nb, block), block, 0, s>>>(nb, count, tiles, ctrl, n);
-    // the records lie in the columns' scratch (108 bytes a particle, of which they
-    // take 80 or 64), on a 16-byte boundary whatever the caller's scratch is on
-    void* records = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(base + L.tmp64) + 15) & ~(uintptr_t)15);
+    uint4* records = records_in(base, L);
     if (st->precision == PPT_PREC_F64) permute<true>(st, key, count, ctrl, order, rf_phase, records, s);
     else permute<false>(st, key, count, ctrl, order, rf_phase, records, s);
     PPT_CUDA_TRY(cudaGetLastError());
@@ -413,29 +401,10 @@ extern "C" int ppt_restore_order(ppt_state* st, int64_t* order, double* rf_phase
     if (st->n == 0) return PPT_OK;
     if (!order || !scratch) return fail(PPT_ERR_ARG, "order and scratch must not be NULL");
     const int64_t n = st->n;
-    SortLayout L = sort_layout(n);
-    char* base = static_cast<char*>(scratch);
-    double* tmp64 = reinterpret_cast<double*>(base + L.tmp64);
-    uint32_t* tmp32 = reinterpret_cast<uint32_t*>(base + L.tmp32);
-    double* phase_tmp = reinterpret_cast<double*>(base + L.phase);
-    uint32_t* perm = reinterpret_cast<uint32_t*>(base + L.perm);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int block = 256;
-    PPT_CUDA_TRY(cudaMemsetAsync(perm, 0xff, (size_t)n * 4, s));   // unclaimed positions: skipped
-    restore_inverse<<<grid_for(n, block), block, 0, s>>>(n, order, perm);
-    if (st->precision == PPT_PREC_F64) {
-        restore_gather<<<grid_for(n, block), block, 0, s>>>(n, perm, 6, st->f64, tmp64, 0, nullptr, 0, nullptr,
-                                                            nullptr, rf_phase, phase_tmp);
-        PPT_CUDA_TRY(cudaMemcpyAsync(st->f64, tmp64, (size_t)n * 6 * 8, cudaMemcpyDeviceToDevice, s));
-    } else {
-        restore_gather<<<grid_for(n, block), block, 0, s>>>(
-            n, perm, 0, nullptr, nullptr, 3, reinterpret_cast<const uint32_t*>(st->i32), 12,
-            reinterpret_cast<const uint32_t*>(st->f32), tmp32, rf_phase, phase_tmp);
-        PPT_CUDA_TRY(cudaMemcpyAsync(st->i32, tmp32, (size_t)n * 3 * 4, cudaMemcpyDeviceToDevice, s));
-        PPT_CUDA_TRY(cudaMemcpyAsync(st->f32, tmp32 + 3 * n, (size_t)n * 12 * 4, cudaMemcpyDeviceToDevice, s));
-    }
-    if (rf_phase) PPT_CUDA_TRY(cudaMemcpyAsync(rf_phase, phase_tmp, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
-    iota_rows<<<grid_for(n, block), block, 0, s>>>(n, order);
+    uint4* records = records_in(static_cast<char*>(scratch), sort_layout(n));
+    if (st->precision == PPT_PREC_F64) permute<true>(st, nullptr, nullptr, nullptr, order, rf_phase, records, s);
+    else permute<false>(st, nullptr, nullptr, nullptr, order, rf_phase, records, s);
     PPT_CUDA_TRY(cudaGetLastError());
     return PPT_OK;
 }

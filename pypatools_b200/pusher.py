@@ -351,8 +351,8 @@ class DeviceTracker:
                                               self.rf_phase.data_ptr() if self.rf_phase is not None else None,
                                               scratch.data_ptr(), self._stream(stream)))
         self.row_order = True
-        # inverse, gather and iota kernels (the fill and copy-backs are memset / memcpy calls)
-        self.launches += 3
+        # scatter, unpack
+        self.launches += 2
 
     def sort(self, stream=None):
         """Reorder particles by cell (gather locality)."""
