@@ -337,7 +337,8 @@ int ppt_jobs_destroy(ppt_jobs* jobs);
  * device: the permutation runs when at least n/16 particles are inside the
  * map, or when the warps holding in-map particles exceed the ones they need
  * by n/512; otherwise the call is a no-op that never waits on the host.
- * scratch: device buffer of ppt_cell_sort_scratch_bytes(n) bytes. */
+ * scratch: device buffer of ppt_cell_sort_scratch_bytes(n) bytes, on an 8-byte
+ * boundary at least. */
 int64_t ppt_cell_sort_scratch_bytes(int64_t n);
 int ppt_cell_sort(ppt_state* st, const ppt_fields* fields, int64_t* order, double* rf_phase,
                   void* scratch, void* stream);

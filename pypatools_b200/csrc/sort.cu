@@ -5,8 +5,9 @@
 // Counting sort on the particle's map-0 cell: bucket = linear cell index
 // (k fastest) modulo 2^22 -- exact for maps up to 4M cells, a hash beyond;
 // particles outside the map share one last bucket.  Histogram -> exclusive
-// scan -> scatter into a scratch copy -> copy back, with warp-aggregated
-// atomics (lanes with equal keys combine before touching memory).  The
+// scan -> scatter of whole slots as records -> records back into columns, with
+// warp-aggregated atomics (lanes with equal keys combine before touching
+// memory).  The
 // reordering runs when at least 1/16 of the particles are inside the map, or
 // when the warps holding in-map particles exceed the ones those particles
 // need by n/512 (a few particles still in the map after the bunch has left,
