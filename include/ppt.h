@@ -377,7 +377,9 @@ int ppt_deposit_cic(int64_t n, const double* r, const double* q, const ppt_mesh_
  * rhs, phi, ex, ey, ez are device (nx, ny, nz) float64 arrays.
  * ppt_poisson_solve: conjugate gradients, matrix-free, from the initial guess
  * in phi until |r| <= rel_tol |rhs| or max_iter iterations; synchronises the
- * stream a few times; reports the iterations and the final |r| / |rhs|.
+ * stream a few times; reports the iterations and the final |r| / |rhs|.  After
+ * PPT_ERR_TIMEOUT (a bounded wait between the solve's blocks ran out) parts of phi
+ * may hold the solve's result and others the guess: start again from a new one.
  * ppt_field_from_potential: central differences at cells whose three indices
  * are interior, 0 on the outer layer (any of ex, ey, ez may be NULL). */
 int64_t ppt_poisson_scratch_bytes(const ppt_mesh_desc* mesh);

@@ -371,6 +371,7 @@ constexpr int kResMaxCg = 12;     // cells per thread: x, A r and A p in registe
 constexpr int kResMaxBi = 8;      // r, t, v and x in registers
 constexpr int kResMaxSums = 5;
 constexpr int kSpinLimit = 1 << 21;   // polls of one wait (~0.5 us each) before the solve gives up
+constexpr unsigned long long kGaveUp = ~0ull;   // in place of a wait's number: block 0 gave it up
 
 // A partial sum and the number of the wait it belongs to, written and read as
 // one 128-bit access.
@@ -383,10 +384,10 @@ struct alignas(16) Slot {
 // the grid's: slots[(e & 1) * kResMaxSums * (blocks + 1) + ...].
 constexpr int kSlotsPerBlock = 4 * kResMaxSums;   // two waits, and as much again: at least two blocks
 
-// What a solve reports, written once at its end (`finished` stays 0 when a
-// wait ran out).
+// What a solve reports: written by block 0 at its end (`finished` stays 0 when
+// it left before), and `late` by every block that gave up a wait.
 struct ResidentOut {
-    double rr, bb, iterations, finished;
+    double rr, bb, iterations, finished, late;
 };
 
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
@@ -434,15 +435,20 @@ __device__ __forceinline__ double warp_sums(const double (&a)[W], int lane, int 
 
 // Wait number e of the grid: each of the N values summed over all threads of
 // all blocks, the same bits in every block; everything the blocks wrote before
-// the call is visible after it.  False when the wait ran out (then every block
-// leaves its solve).  Block 0 gathers the partial sums and hands out the grid's,
+// the call is visible after it.  False when the wait ran out after `polls` polls:
+// then the block leaves its solve and says so in out->late, which is an error of
+// the whole solve.  Block 0 passes a wait that it gave up on to every block
+// (kGaveUp in place of the sum), so none goes on with a sum of some of them; a
+// block that gives up by itself leaves block 0 to give up the next wait.
+// Block 0 gathers the partial sums and hands out the grid's,
 // each as one 16-byte word with the step's number.  With every block reading
 // all partial sums instead, a step among 148 blocks takes 4.1 us for one value,
 // 6.3 for two and 7.2 for five, since their polls of the same lines hold up one
 // another and the stores they wait for; so it takes 3.1 and 3.2 us for one and
 // for four.
 template <int N>
-__device__ __forceinline__ bool grid_sums(Slot* slots, GridSums& G, unsigned long long e, double (&a)[N]) {
+__device__ __forceinline__ bool grid_sums(Slot* slots, ResidentOut* out, int polls, GridSums& G, unsigned long long e,
+                                          double (&a)[N]) {
     constexpr int W = sums_width(N);
     constexpr int L = 32 / W;                   // lanes of one value
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -485,22 +491,30 @@ __device__ __forceinline__ bool grid_sums(Slot* slots, GridSums& G, unsigned lon
                 all = true;
 #pragma unroll
                 for (int u = 0; u < kPolls; ++u) all = all && when[u] == e;
-            } while (!all && ++spins < kSpinLimit);
-            if (!all) G.late = 1;
-            fence_gpu();          // what the blocks wrote before their words is passed on with the sum
+            } while (!all && ++spins < polls);
+            fence_gpu();          // a lane sees what the blocks whose words it polled wrote before them
             v = 0.0;
 #pragma unroll
             for (int u = 0; u < kPolls; ++u) v += lane + 32 * u < nb ? got[u] : 0.0;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) publish(down + warp - 1, v, e);
+            const bool whole = __all_sync(0xffffffffu, all);
+            // and lane 0 passes it on with the sum: the shuffles order no memory, so the
+            // lanes' reads come before its word by the barrier and a fence of its own
+            __syncwarp();
+            if (lane == 0) {
+                fence_gpu();
+                publish(down + warp - 1, v, whole ? e : kGaveUp);
+            }
         }
         if (warp == 0) {
             if (lane < N) {
                 double sum;
                 int spins = 0;
-                while (poll(down + lane, sum) != e && ++spins < kSpinLimit) {}
-                if (spins >= kSpinLimit) G.late = 1;
+                unsigned long long when;
+                do when = poll(down + lane, sum);
+                while (when != e && when != kGaveUp && ++spins < polls);
+                if (when != e) G.late = 1;
                 G.all[lane] = sum;
             }
             fence_gpu();          // what the blocks wrote before the wait is read after it
@@ -509,7 +523,9 @@ __device__ __forceinline__ bool grid_sums(Slot* slots, GridSums& G, unsigned lon
     __syncthreads();
 #pragma unroll
     for (int n = 0; n < N; ++n) a[n] = G.all[n];
-    return G.late == 0;
+    if (G.late == 0) return true;
+    if (threadIdx.x == 0) out->late = 1.0;
+    return false;
 }
 
 // The bricks: b[d] cells along axis d, the last ones fewer; g[d] of them.
@@ -641,7 +657,7 @@ template <int S>
 __global__ void __launch_bounds__(kResThreads, 1)
     cg_resident(const __grid_constant__ PoissonOp A, const __grid_constant__ Bricks B, const double* __restrict__ rhs,
                 double* x_out, double* w_pub, int64_t m, Slot* slots, ResidentOut* out, double rel_tol,
-                int64_t max_iter) {
+                int64_t max_iter, int polls) {
     extern __shared__ double shared[];
     __shared__ GridSums G;
     __shared__ int count;
@@ -679,7 +695,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     }
     for (int h = threadIdx.x; h < P.halo; h += kResThreads) halo_q[h] = 0.0;
     unsigned long long epoch = 1;
-    if (!grid_sums(slots, G, epoch, first)) return;
+    if (!grid_sums(slots, out, polls, G, epoch, first)) return;
 #pragma unroll
     for (int s = 0; s < S; ++s)                    // the padded brick held x; now r
         if (own[s] & kOwned) r[own[s] & 0xffff] = w[s];
@@ -703,7 +719,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             sum[0] = fma(rc, rc, sum[0]);
             sum[1] = fma(w[s], rc, sum[1]);
         }
-        if (!grid_sums(slots, G, ++epoch, sum)) return;
+        if (!grid_sums(slots, out, polls, G, ++epoch, sum)) return;
         rr = sum[0];
         if (rr <= tol2 || rr == 0.0 || it >= max_iter) break;
         const double beta = it == 0 ? 0.0 : rr / rr_old;
@@ -733,7 +749,12 @@ __global__ void __launch_bounds__(kResThreads, 1)
             x_out[c] = x[s];
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *out = ResidentOut{rr, bb, (double)it, 1.0};
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out->rr = rr;
+        out->bb = bb;
+        out->iterations = (double)it;
+        out->finished = 1.0;
+    }
 }
 
 // What a cell's coefficient row is, decided once per solve: most rows are the
@@ -791,7 +812,7 @@ template <int S>
 __global__ void __launch_bounds__(kResThreads, 1)
     bi_resident(const __grid_constant__ PoissonOp A, const __grid_constant__ Bricks B,
                 const double* __restrict__ coef, const double* __restrict__ rhs, double* x_out, double* v_pub,
-                double* t_pub, int row_space, Slot* slots, ResidentOut* out, double rel_tol, int64_t max_iter) {
+                double* t_pub, int row_space, Slot* slots, ResidentOut* out, double rel_tol, int64_t max_iter, int polls) {
     extern __shared__ double shared[];
     __shared__ GridSums G;
     __shared__ int count, n_rows;
@@ -870,7 +891,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         if (__all_sync(0xffffffffu, row[s] == 63)) own[s] |= kPlainWarp;
     }
     unsigned long long epoch = 1;
-    if (!grid_sums(slots, G, epoch, first)) return;
+    if (!grid_sums(slots, out, polls, G, epoch, first)) return;
     update_halo(P, t_pub, [&](int h, int, double rc) { halo_r[h] = rc; });
     double rr = first[0], rho = rr, beta = 0.0, omega = 1.0;
     double rhat2 = rr;                 // |rhat|^2
@@ -910,7 +931,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 rhat[threadIdx.x + s * kResThreads] = r[s];
                 sum[0] = fma(r[s], r[s], sum[0]);
             }
-            if (!grid_sums(slots, G, ++epoch, sum)) return;
+            if (!grid_sums(slots, out, polls, G, ++epoch, sum)) return;
             rr = rho = rhat2 = sum[0];
             if (rr <= tol2 || rr == 0.0) break;
             fresh = true;
@@ -939,7 +960,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             if (own[s] & kFace) v_pub[K.base + l] = v[s];
             dv[0] = fma(rhat[l], v[s], dv[0]);           // rhat is zero past the brick's cells
         }
-        if (!grid_sums(slots, G, ++epoch, dv)) return;
+        if (!grid_sums(slots, out, polls, G, ++epoch, dv)) return;
         if (dv[0] == 0.0) {
             restart = true;
             done = ++it >= max_iter;
@@ -974,7 +995,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             sum[3] = fma(rhat[l], t[s], sum[3]);
             sum[4] = fma(r[s], r[s], sum[4]);
         }
-        if (!grid_sums(slots, G, ++epoch, sum)) return;
+        if (!grid_sums(slots, out, polls, G, ++epoch, sum)) return;
         omega = sum[1] > 0.0 ? sum[0] / sum[1] : 0.0;
         // x += alpha p^ + omega s^, r = s - omega t
         update_halo(P, t_pub, [&](int h, int, double tc) { halo_r[h] = fma(-omega, tc, halo_r[h]); });
@@ -1003,7 +1024,12 @@ __global__ void __launch_bounds__(kResThreads, 1)
             x_out[c] = x[s];
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *out = ResidentOut{rr, bb, (double)it, 1.0};
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out->rr = rr;
+        out->bb = bb;
+        out->iterations = (double)it;
+        out->finished = 1.0;
+    }
 }
 
 // The bricks of a resident solve, its cells per thread (0: the mesh does not
@@ -1017,12 +1043,13 @@ struct ResidentPlan {
     size_t smem;
     Slot* slots;
     ResidentOut* out;
+    int polls;         // of a grid-wide wait, at most
 };
 
 constexpr size_t kResSharedLimit = 224 * 1024;   // with the static arrays below the 227 KB of a block
 
 static cudaError_t plan_resident(const int64_t n[3], int most, int padded_vectors, int plain_vectors,
-                                 int face_vectors, double* spare, double* sums, ResidentPlan* plan) {
+                                 int face_vectors, double* spare, double* sums, int polls, ResidentPlan* plan) {
     plan->per_thread = 0;
     int dev = 0, sms = 0, coop = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1069,6 +1096,7 @@ static cudaError_t plan_resident(const int64_t n[3], int most, int padded_vector
     static_assert(sizeof(ResidentOut) <= 9 * sizeof(double), "the report fits the sums' scratch");
     plan->slots = reinterpret_cast<Slot*>((reinterpret_cast<uintptr_t>(spare) + 15) & ~(uintptr_t)15);
     plan->out = reinterpret_cast<ResidentOut*>(sums);
+    plan->polls = polls;
     return cudaSuccess;
 }
 
@@ -1083,7 +1111,7 @@ static int run_resident(const void* kernel, const ResidentPlan& plan, void** arg
     ResidentOut host;
     PPT_CUDA_TRY(cudaMemcpyAsync(&host, plan.out, sizeof(host), cudaMemcpyDeviceToHost, s));
     PPT_CUDA_TRY(cudaStreamSynchronize(s));
-    if (host.finished != 1.0) return fail(PPT_ERR_TIMEOUT, "a grid-wide wait of the solver ran out");
+    if (host.finished != 1.0 || host.late != 0.0) return fail(PPT_ERR_TIMEOUT, "a grid-wide wait of the solver ran out");
     if (iterations) *iterations = (int64_t)host.iterations;
     if (rel_residual) *rel_residual = host.bb > 0.0 ? std::sqrt(host.rr / host.bb) : 0.0;
     return PPT_OK;
@@ -1173,9 +1201,8 @@ extern "C" int64_t ppt_poisson_scratch_bytes(const ppt_mesh_desc* mesh) {
     return (3 * m + 2 * nb + kNumScalars) * (int64_t)sizeof(double);
 }
 
-extern "C" int ppt_poisson_solve(const ppt_mesh_desc* mesh, const double* rhs, double* phi, void* scratch,
-                                 double rel_tol, int64_t max_iter, int64_t* iterations, double* rel_residual,
-                                 void* stream) {
+static int solve_laplacian(const ppt_mesh_desc* mesh, const double* rhs, double* phi, void* scratch, double rel_tol,
+                           int64_t max_iter, int polls, int64_t* iterations, double* rel_residual, void* stream) {
     int64_t n[3];
     double h[3];
     int rc = mesh_geom(mesh, n, h);
@@ -1194,11 +1221,12 @@ extern "C" int ppt_poisson_solve(const ppt_mesh_desc* mesh, const double* rhs, d
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     double host[kNumScalars];
     ResidentPlan plan;
-    PPT_CUDA_TRY(plan_resident(n, kResMaxCg, 1, 1, 1, q, part, &plan));
+    PPT_CUDA_TRY(plan_resident(n, kResMaxCg, 1, 1, 1, q, part, polls, &plan));
     if (plan.per_thread) {
         int64_t mm = m;
         double* w_pub = r;            // two buffers; q is left for the slots
-        void* args[] = {&A, &plan.bricks, &rhs, &phi, &w_pub, &mm, &plan.slots, &plan.out, &rel_tol, &max_iter};
+        void* args[] = {&A,   &plan.bricks, &rhs,      &phi,      &w_pub,
+                        &mm,  &plan.slots,  &plan.out, &rel_tol,  &max_iter, &plan.polls};
         const void* kernel = plan.per_thread == 1   ? (const void*)cg_resident<1>
                              : plan.per_thread == 2 ? (const void*)cg_resident<2>
                              : plan.per_thread == 4 ? (const void*)cg_resident<4>
@@ -1224,6 +1252,12 @@ extern "C" int ppt_poisson_solve(const ppt_mesh_desc* mesh, const double* rhs, d
     return PPT_OK;
 }
 
+extern "C" int ppt_poisson_solve(const ppt_mesh_desc* mesh, const double* rhs, double* phi, void* scratch,
+                                 double rel_tol, int64_t max_iter, int64_t* iterations, double* rel_residual,
+                                 void* stream) {
+    return solve_laplacian(mesh, rhs, phi, scratch, rel_tol, max_iter, kSpinLimit, iterations, rel_residual, stream);
+}
+
 extern "C" int ppt_field_from_potential(const ppt_mesh_desc* mesh, const double* phi, double* ex, double* ey,
                                         double* ez, void* stream) {
     int64_t n[3];
@@ -1247,9 +1281,9 @@ extern "C" int64_t ppt_poisson_coef_scratch_bytes(const ppt_mesh_desc* mesh) {
     return (6 * m + 2 * nb + bNumScalars) * (int64_t)sizeof(double);
 }
 
-extern "C" int ppt_poisson_solve_coef(const ppt_mesh_desc* mesh, const double* coef, const double* rhs, double* phi,
-                                      void* scratch, double rel_tol, int64_t max_iter, int64_t* iterations,
-                                      double* rel_residual, void* stream) {
+static int solve_coef(const ppt_mesh_desc* mesh, const double* coef, const double* rhs, double* phi, void* scratch,
+                      double rel_tol, int64_t max_iter, int polls, int64_t* iterations, double* rel_residual,
+                      void* stream) {
     int64_t n[3];
     double h[3];
     int rc = mesh_geom(mesh, n, h);
@@ -1273,7 +1307,7 @@ extern "C" int ppt_poisson_solve_coef(const ppt_mesh_desc* mesh, const double* c
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     double host[bNumScalars];
     ResidentPlan plan;
-    PPT_CUDA_TRY(plan_resident(n, kResMaxBi, 2, 1, 4, p, part, &plan));
+    PPT_CUDA_TRY(plan_resident(n, kResMaxBi, 2, 1, 4, p, part, polls, &plan));
     if (plan.per_thread) {
         PoissonOp L = laplacian(n, h);
         double* v_pub = r;
@@ -1282,8 +1316,8 @@ extern "C" int ppt_poisson_solve_coef(const ppt_mesh_desc* mesh, const double* c
         int row_space = (int)((kResSharedLimit - plan.smem) / sizeof(Row));
         if (row_space > plan.per_thread * kResThreads + kFixedRows) row_space = plan.per_thread * kResThreads + kFixedRows;
         plan.smem += (size_t)row_space * sizeof(Row);
-        void* args[] = {&L,     &plan.bricks, &coef,       &rhs,      &phi,     &v_pub,
-                        &t_pub, &row_space,   &plan.slots, &plan.out, &rel_tol, &max_iter};
+        void* args[] = {&L,         &plan.bricks, &coef,     &rhs,     &phi,      &v_pub,     &t_pub, &row_space,
+                        &plan.slots, &plan.out,   &rel_tol, &max_iter, &plan.polls};
         const void* kernel = plan.per_thread == 1   ? (const void*)bi_resident<1>
                              : plan.per_thread == 2 ? (const void*)bi_resident<2>
                              : plan.per_thread == 4 ? (const void*)bi_resident<4>
@@ -1307,4 +1341,18 @@ extern "C" int ppt_poisson_solve_coef(const ppt_mesh_desc* mesh, const double* c
     if (iterations) *iterations = (int64_t)host[bITERS];
     if (rel_residual) *rel_residual = host[bBB] > 0.0 ? std::sqrt(host[bRR] / host[bBB]) : 0.0;
     return PPT_OK;
+}
+
+extern "C" int ppt_poisson_solve_coef(const ppt_mesh_desc* mesh, const double* coef, const double* rhs, double* phi,
+                                      void* scratch, double rel_tol, int64_t max_iter, int64_t* iterations,
+                                      double* rel_residual, void* stream) {
+    return solve_coef(mesh, coef, rhs, phi, scratch, rel_tol, max_iter, kSpinLimit, iterations, rel_residual, stream);
+}
+
+// The two solves (coef NULL: the first) with waits of at most `polls` polls:
+// how a test makes one run out.  Not part of the library's interface.
+extern "C" int ppt_poisson_solve_polls(const ppt_mesh_desc* mesh, const double* coef, const double* rhs, double* phi,
+                                       void* scratch, double rel_tol, int64_t max_iter, int polls, void* stream) {
+    if (coef) return solve_coef(mesh, coef, rhs, phi, scratch, rel_tol, max_iter, polls, nullptr, nullptr, stream);
+    return solve_laplacian(mesh, rhs, phi, scratch, rel_tol, max_iter, polls, nullptr, nullptr, stream);
 }
