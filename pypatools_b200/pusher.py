@@ -481,10 +481,13 @@ class HostStager:
     def __init__(self, device, chunk=2 << 20, slots=96, threads=None):
         import ctypes
         import os
+        import threading
         torch = _torch()
         self.torch = torch
         self.device = device
         self.lib = _lib.load()
+        self._copies = []               # the downloads whose memory is in use: [src, dst, queued]
+        self._copies_lock = threading.Lock()
         if threads is None:
             threads = max(1, min(12, (os.cpu_count() or 8) - 2))
         self.stream = torch.cuda.Stream(device=device)
@@ -505,13 +508,21 @@ class HostStager:
     def copy(self, src, dst, after=None):
         """Queue the copy of the contiguous device tensor ``src`` into the
         contiguous numpy array ``dst`` (same bytes), after event ``after``.
-        The caller keeps ``src`` alive (and unchanged) until ``finish()``
-        returns: the copy stream reads it after this call returns."""
+        The caller keeps ``src`` unchanged until ``finish()`` returns: the copy
+        stream reads it after this call returns.  Both are referenced until then,
+        so a caller that never gets to ``finish`` drops neither of them under the
+        copy; a later ``finish`` of any thread lets go of them."""
         nbytes = src.numel() * src.element_size()
         if nbytes != dst.nbytes or not src.is_contiguous() or not dst.flags.c_contiguous:
             raise ValueError("src and dst must be contiguous and of the same size")
-        _lib.check(self.lib.ppt_stager_download(self.handle, dst.ctypes.data, src.data_ptr(), nbytes,
-                                                after.cuda_event if after is not None else None))
+        entry = [src, dst, False]
+        with self._copies_lock:
+            self._copies.append(entry)
+        try:
+            _lib.check(self.lib.ppt_stager_download(self.handle, dst.ctypes.data, src.data_ptr(), nbytes,
+                                                    after.cuda_event if after is not None else None))
+        finally:
+            entry[2] = True             # the next finish waits for what was queued of it
 
     def upload(self, src, dst, stream=None):
         """Copy the contiguous numpy array ``src`` into the contiguous device
@@ -525,8 +536,14 @@ class HostStager:
         _lib.check(self.lib.ppt_stager_upload(self.handle, dst.data_ptr(), src.ctypes.data, nbytes, st.cuda_stream))
 
     def finish(self):
-        """Wait until every copy queued so far is in its numpy array."""
-        _lib.check(self.lib.ppt_stager_finish(self.handle))
+        """Wait until every copy queued so far is in its numpy array; raises what
+        went wrong with one of the calling thread."""
+        with self._copies_lock:
+            landed = {id(c) for c in self._copies if c[2]}
+        rc = self.lib.ppt_stager_finish(self.handle)
+        with self._copies_lock:
+            self._copies = [c for c in self._copies if id(c) not in landed]
+        _lib.check(rc)
 
 
 class PusherGPU:
@@ -721,10 +738,15 @@ class PusherGPU:
                     # the closing half step of the Boris family
                     drain(min(done // rec + 1, n_rec - 1))
 
-            tr.run(nsteps, chunk, sort_every=sort_every, after_launch=after_launch)
-            if to_host:
-                drain(n_rec)
-                stager.finish()
+            try:
+                tr.run(nsteps, chunk, sort_every=sort_every, after_launch=after_launch)
+                if to_host:
+                    drain(n_rec)
+            finally:
+                # also when a launch, a print or Ctrl-C ends the track: its rows are
+                # still on their way into h_r and h_v
+                if to_host:
+                    stager.finish()
             status = tr.device_status()
         if status & _lib.STATUS_NONFINITE:
             warnings.warn("non-finite particle state encountered during tracking", RuntimeWarning)

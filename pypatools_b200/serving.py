@@ -256,9 +256,11 @@ class TrackingServer:
         def work():
             r = host_array(tuple(tr.r_hist.shape))
             v = host_array(tuple(tr.v_hist.shape))
-            stager.copy(tr.r_hist, r)
-            stager.copy(tr.v_hist, v)
-            stager.finish()
+            try:
+                stager.copy(tr.r_hist, r)
+                stager.copy(tr.v_hist, v)
+            finally:
+                stager.finish()
             return r, v, time.perf_counter() - t_base
 
         return self._pool.submit(work)

@@ -1,0 +1,81 @@
+"""The staging of host copies without a GPU: the Python side's references."""
+import weakref
+
+import numpy as np
+import pytest
+
+
+class _FakeLib:
+    def __init__(self):
+        self.finished = 0
+
+    def ppt_stager_download(self, *a):
+        return 0
+
+    def ppt_stager_finish(self, handle):
+        self.finished += 1
+        return 0
+
+
+def _stager():
+    import threading
+    from pypatools_b200.pusher import HostStager
+    st = object.__new__(HostStager)
+    st.lib, st.handle, st._copies, st._copies_lock = _FakeLib(), 1, [], threading.Lock()
+    return st
+
+
+def test_a_copy_keeps_both_ends_until_finish():
+    import torch
+    st = _stager()
+    src, dst = torch.zeros(10, dtype=torch.float64), np.empty(10)
+    ends = weakref.ref(src), weakref.ref(dst)
+    st.copy(src, dst)
+    del src, dst
+    assert all(r() is not None for r in ends)
+    st.finish()
+    assert all(r() is None for r in ends)
+
+
+def test_an_interrupted_track_waits_for_its_rows(monkeypatch):
+    """A track that ends with an exception after rows were queued."""
+    import contextlib
+    import torch
+    from pypatools_b200 import IonSpecies, pusher
+    st = _stager()
+
+    class Tracker:
+        active = None
+
+        def __init__(self, alg, qm, df, m, nsteps, dt, rec, *a, **k):
+            self.r_hist = torch.zeros((nsteps // rec + 1, m, 3), dtype=torch.float64)
+            self.v_hist = self.r_hist.clone()
+
+        def load(self, r, v):
+            pass
+
+        def run(self, nsteps, chunk, sort_every=0, after_launch=None):
+            after_launch(nsteps // 2)
+            raise KeyboardInterrupt
+
+    class Fields:
+        device = torch.device("cpu")
+
+    class Event:
+        cuda_event = 0
+
+        def record(self, stream):
+            pass
+
+    monkeypatch.setattr(pusher, "DeviceTracker", Tracker)
+    monkeypatch.setattr(pusher, "_torch", lambda: torch)
+    monkeypatch.setattr(pusher.HostStager, "for_device", classmethod(lambda cls, device: st))
+    monkeypatch.setattr(pusher.PusherGPU, "_device_fields", lambda self, e, b: Fields)
+    monkeypatch.setattr(pusher.PusherGPU, "_upload", staticmethod(lambda a, device: torch.from_numpy(a)))
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: None)
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    p = pusher.PusherGPU(IonSpecies("proton"), "boris")
+    with pytest.raises(KeyboardInterrupt):
+        p.track_batch(np.zeros((5, 3)), np.ones((5, 3)), None, None, 10, 1e-10)
+    assert st.lib.finished == 1 and not st._copies
