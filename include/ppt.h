@@ -445,7 +445,8 @@ int ppt_stager_upload(ppt_stager* s, void* dst, const void* src, int64_t bytes, 
 
 /* Device src -> host dst, queued, once the cudaEvent_t `after` has happened
  * (NULL: at once).  src must stay as it is, and dst is complete, when
- * ppt_stager_finish returns. */
+ * ppt_stager_finish returns (or when this call returns an error: then nothing of
+ * it is in flight). */
 int ppt_stager_download(ppt_stager* s, void* dst, const void* src, int64_t bytes, void* after);
 
 /* Wait for every download queued before the call. */

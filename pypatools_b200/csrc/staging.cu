@@ -21,7 +21,6 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
-#include <deque>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -86,6 +85,20 @@ struct StagerLanding {
     bool stream;
 };
 
+// A queue of landings that never allocates: a slot is in it at most once.
+struct StagerQueue {
+    std::vector<StagerLanding> at;
+    size_t first = 0, count = 0;
+    bool empty() const { return count == 0; }
+    void push(const StagerLanding& t) { at[(first + count++) % at.size()] = t; }
+    StagerLanding pop() {
+        const StagerLanding t = at[first];
+        first = (first + 1) % at.size();
+        --count;
+        return t;
+    }
+};
+
 struct StagerSleeper {
     sem_t sem;
     std::atomic<bool> asleep{false};
@@ -118,8 +131,8 @@ struct ppt_stager {
     std::mutex ring;                        // one upload or download is being cut into pieces at a time
     ppt::StagerUpload up;
     std::mutex m;                           // the fields below and the slots' busy and seq
-    std::deque<ppt::StagerLanding> arriving;   // device -> slot, in the order of the copies
-    std::deque<ppt::StagerLanding> land;       // slot -> host
+    ppt::StagerQueue arriving;              // device -> slot, in the order of the copies
+    ppt::StagerQueue land;                  // slot -> host
     std::condition_variable arrival, done;
     // The pool joins without the mutex: threads woken one after the other through
     // it would queue for it.  A thread counts itself into `joined` before it looks
@@ -172,15 +185,14 @@ static void stager_waiter(ppt_stager* S) {
             std::unique_lock<std::mutex> lock(S->m);
             S->arrival.wait(lock, [&] { return S->stop_waiter || !S->arriving.empty(); });
             if (S->arriving.empty()) return;
-            t = S->arriving.front();
-            S->arriving.pop_front();
+            t = S->arriving.pop();
         }
         const cudaError_t e = cudaEventSynchronize(S->slots[t.slot].ev);
         const bool small = t.bytes <= kMinPiece;       // not worth handing over
         if (e == cudaSuccess && small) copy_bytes(t.host, S->slots[t.slot].buf, t.bytes, t.stream);
         std::lock_guard<std::mutex> lock(S->m);
         if (e == cudaSuccess && !small) {
-            S->land.push_back(t);
+            S->land.push(t);
             S->landings.fetch_add(1);
             wake(S, 1);
         } else {
@@ -207,8 +219,7 @@ static void stager_worker(ppt_stager* S, int me) {
             {
                 std::lock_guard<std::mutex> lock(S->m);
                 if (!S->land.empty()) {
-                    t = S->land.front();
-                    S->land.pop_front();
+                    t = S->land.pop();
                     S->landings.fetch_sub(1);
                     have = true;
                 }
@@ -315,10 +326,23 @@ static cudaError_t download(ppt_stager* S, char* dst, const char* src, int64_t b
         std::lock_guard<std::mutex> lock(S->m);
         slot.busy = true;
         slot.seq = ++S->queued;
-        S->arriving.push_back(StagerLanding{k, dst + a, b - a, bytes > kStreamBytes});
+        S->arriving.push(StagerLanding{k, dst + a, b - a, bytes > kStreamBytes});
         S->arrival.notify_one();
     }
     return cudaSuccess;
+}
+
+// After an error, with S->ring held: nothing of the call is in flight any more
+// (downloads beyond the first `before`, an upload's copies), so the caller may
+// give its memory back.
+static void settle(ppt_stager* S, uint64_t before) {
+    cudaStreamSynchronize(S->stream);
+    std::unique_lock<std::mutex> lock(S->m);
+    S->done.wait(lock, [&] {
+        for (const StagerSlot& s : S->slots)
+            if (s.busy && s.seq > before) return false;
+        return true;
+    });
 }
 
 // The stager's device is current while one of its calls runs.
@@ -373,6 +397,8 @@ extern "C" int ppt_stager_create(int64_t slot_bytes, int n_slots, int n_threads,
     try {
         S = new ppt_stager;
         S->slots.resize((size_t)n_slots);
+        S->arriving.at.resize((size_t)n_slots);
+        S->land.at.resize((size_t)n_slots);
         S->slot_bytes = slot_bytes;
         S->stream = static_cast<cudaStream_t>(copy_stream);
         cudaError_t e = cudaGetDevice(&S->device);
@@ -413,6 +439,7 @@ extern "C" int ppt_stager_upload(ppt_stager* S, void* dst, const void* src, int6
         if (e == cudaSuccess) e = upload(S, static_cast<char*>(dst), static_cast<const char*>(src), bytes);
         if (e == cudaSuccess) e = cudaEventRecord(ev, S->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(user, ev, 0);
+        if (e != cudaSuccess) cudaStreamSynchronize(S->stream);   // dst may go once the call has failed
         cudaEventDestroy(ev);
         return e == cudaSuccess ? PPT_OK : cuda_fail(e, "staged upload");
     } catch (const std::exception& ex) {
@@ -425,8 +452,10 @@ extern "C" int ppt_stager_download(ppt_stager* S, void* dst, const void* src, in
     try {
         std::lock_guard<std::mutex> ring(S->ring);
         OnDevice on(S->device);
+        const uint64_t before = S->queued;
         cudaError_t e = after ? cudaStreamWaitEvent(S->stream, static_cast<cudaEvent_t>(after), 0) : cudaSuccess;
         if (e == cudaSuccess) e = download(S, static_cast<char*>(dst), static_cast<const char*>(src), bytes);
+        if (e != cudaSuccess) settle(S, before);
         return e == cudaSuccess ? PPT_OK : cuda_fail(e, "staged download");
     } catch (const std::exception& ex) {
         return fail(PPT_ERR_OOM, std::string("stager: ") + ex.what());

@@ -1,8 +1,40 @@
-"""The staging of host copies without a GPU: the Python side's references."""
+"""The staging of host copies without a GPU: csrc/staging.cu against a stand-in
+for the CUDA runtime (tests/stager_host), and the Python side's references."""
+import shutil
+import subprocess
 import weakref
+from pathlib import Path
 
 import numpy as np
 import pytest
+
+HERE = Path(__file__).resolve().parent
+REPO = HERE.parent
+
+
+def _compile(folder, *flags):
+    """The cases' program.  staging.cu is copied beside the stand-in, so that
+    its quoted include finds that first."""
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not found")
+    for name in ("ppt_internal.cuh", "main.cpp"):
+        shutil.copy(HERE / "stager_host" / name, folder / name)
+    shutil.copy(REPO / "pypatools_b200" / "csrc" / "staging.cu", folder / "staging.cu")
+    exe = folder / "cases"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-g", *flags, "-I", str(REPO / "include"), str(folder / "main.cpp"),
+                    "-o", str(exe), "-lpthread"], check=True, capture_output=True, text=True)
+    return exe
+
+
+@pytest.fixture(scope="module")
+def cases(tmp_path_factory):
+    return _compile(tmp_path_factory.mktemp("stager"))
+
+
+@pytest.mark.parametrize("case", ["refused_download", "refused_upload", "several_callers"])
+def test_stager(cases, case):
+    res = subprocess.run([str(cases), case], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0, res.stderr
 
 
 class _FakeLib:
