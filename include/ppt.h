@@ -449,7 +449,8 @@ int ppt_stager_upload(ppt_stager* s, void* dst, const void* src, int64_t bytes, 
  * it is in flight). */
 int ppt_stager_download(ppt_stager* s, void* dst, const void* src, int64_t bytes, void* after);
 
-/* Wait for every download queued before the call. */
+/* Wait for every download queued before the call.  An error is one of the
+ * calling thread's own downloads since its last finish. */
 int ppt_stager_finish(ppt_stager* s);
 
 int ppt_stager_destroy(ppt_stager* s);

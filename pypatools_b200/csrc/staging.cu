@@ -21,6 +21,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -83,6 +84,7 @@ struct StagerLanding {
     char* host;
     int64_t bytes;
     bool stream;
+    std::thread::id caller;
 };
 
 // A queue of landings that never allocates: a slot is in it at most once.
@@ -145,7 +147,8 @@ struct ppt_stager {
     bool stop_waiter = false;
     size_t next = 0;
     uint64_t queued = 0;                    // download pieces so far
-    cudaError_t error = cudaSuccess;
+    cudaError_t lost_error = cudaSuccess;
+    std::map<std::thread::id, cudaError_t> errors;   // of the downloads of each caller, until its finish
 };
 
 namespace ppt {
@@ -175,6 +178,16 @@ static void wake(ppt_stager* S, int count) {
         }
 }
 
+// The first error among a caller's downloads; with S->m held.  (Without the
+// memory to note it, it is everyone's: see ppt_stager_finish.)
+static void note_error(ppt_stager* S, std::thread::id caller, cudaError_t e) {
+    try {
+        S->errors.emplace(caller, e);
+    } catch (const std::exception&) {
+        S->lost_error = e;
+    }
+}
+
 // Downloads' copies finish in order: one thread waits for them, so that no
 // thread of the pool is held by the GPU.
 static void stager_waiter(ppt_stager* S) {
@@ -196,7 +209,7 @@ static void stager_waiter(ppt_stager* S) {
             S->landings.fetch_add(1);
             wake(S, 1);
         } else {
-            if (e != cudaSuccess && S->error == cudaSuccess) S->error = e;
+            if (e != cudaSuccess) note_error(S, t.caller, e);
             S->slots[t.slot].busy = false;
             S->done.notify_all();
         }
@@ -326,7 +339,7 @@ static cudaError_t download(ppt_stager* S, char* dst, const char* src, int64_t b
         std::lock_guard<std::mutex> lock(S->m);
         slot.busy = true;
         slot.seq = ++S->queued;
-        S->arriving.push(StagerLanding{k, dst + a, b - a, bytes > kStreamBytes});
+        S->arriving.push(StagerLanding{k, dst + a, b - a, bytes > kStreamBytes, std::this_thread::get_id()});
         S->arrival.notify_one();
     }
     return cudaSuccess;
@@ -472,8 +485,12 @@ extern "C" int ppt_stager_finish(ppt_stager* S) {
                 if (s.busy && s.seq <= upto) return false;
             return true;
         });
-        const cudaError_t e = S->error;
-        S->error = cudaSuccess;
+        cudaError_t e = S->lost_error;
+        const auto mine = S->errors.find(std::this_thread::get_id());
+        if (mine != S->errors.end()) {
+            e = mine->second;
+            S->errors.erase(mine);
+        }
         if (e != cudaSuccess) return cuda_fail(e, "staged copy");
         return PPT_OK;
     } catch (const std::exception& ex) {

@@ -74,6 +74,24 @@ static void refused_upload() {
     expect(in_flight == 0, "its other copies have run");
 }
 
+// A download that fails is an error of the thread that queued it, whoever
+// finishes first.
+static void error_of_its_caller() {
+    Ring ring;
+    std::vector<char> bad(1000, 1), good(1000, 2), a(1000), b(1000);
+    fake_bad_source = bad.data();
+    expect(ppt_stager_download(ring.s, a.data(), bad.data(), 1000, nullptr) == PPT_OK, "queue");
+    int other = -100;
+    std::thread([&] {
+        other = ppt_stager_download(ring.s, b.data(), good.data(), 1000, nullptr);
+        if (other == PPT_OK) other = ppt_stager_finish(ring.s);
+    }).join();
+    expect(other == PPT_OK && b == good, "another thread's download is good");
+    expect(ppt_stager_finish(ring.s) == PPT_ERR_CUDA, "the failed one is reported to its caller");
+    fake_bad_source = nullptr;
+    expect(ppt_stager_finish(ring.s) == PPT_OK, "once");
+}
+
 // Uploads and downloads from several threads: every byte (and, built with
 // -fsanitize=thread, no data race).
 static void several_callers() {
@@ -103,6 +121,7 @@ int main(int argc, char** argv) {
     const std::string which = argc > 1 ? argv[1] : "";
     if (which == "refused_download") refused_download();
     else if (which == "refused_upload") refused_upload();
+    else if (which == "error_of_its_caller") error_of_its_caller();
     else if (which == "several_callers") several_callers();
     else return 2;
     return 0;

@@ -31,7 +31,7 @@ def cases(tmp_path_factory):
     return _compile(tmp_path_factory.mktemp("stager"))
 
 
-@pytest.mark.parametrize("case", ["refused_download", "refused_upload", "several_callers"])
+@pytest.mark.parametrize("case", ["refused_download", "refused_upload", "error_of_its_caller", "several_callers"])
 def test_stager(cases, case):
     res = subprocess.run([str(cases), case], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0, res.stderr
