@@ -114,7 +114,8 @@ struct StagerUpload {
     char* dev = nullptr;
     const char* host = nullptr;
     int64_t bytes = 0, piece = 0;
-    int first = 0, n = 0;                   // slots first, first + 1, ... (around the ring)
+    int first = 0;                          // slots first, first + 1, ... (around the ring)
+    std::atomic<int> n{0};                  // pieces (idle threads look at it while the next upload sets it)
     bool stream = false;
     std::atomic<int> next{0}, done{0};
     std::atomic<int> error{0};

@@ -111,3 +111,16 @@ def test_an_interrupted_track_waits_for_its_rows(monkeypatch):
     with pytest.raises(KeyboardInterrupt):
         p.track_batch(np.zeros((5, 3)), np.ones((5, 3)), None, None, 10, 1e-10)
     assert st.lib.finished == 1 and not st._copies
+
+
+def test_no_data_race(tmp_path):
+    probe = tmp_path / "probe"
+    (tmp_path / "probe.cpp").write_text("int main() { return 0; }\n")
+    built = shutil.which("g++") and subprocess.run(["g++", "-fsanitize=thread", str(tmp_path / "probe.cpp"), "-o",
+                                                    str(probe)], capture_output=True).returncode == 0
+    if not built or subprocess.run([str(probe)], capture_output=True).returncode != 0:
+        pytest.skip("no ThreadSanitizer here")
+    exe = _compile(tmp_path, "-fsanitize=thread")
+    for _ in range(3):
+        res = subprocess.run([str(exe), "several_callers"], capture_output=True, text=True, timeout=300)
+        assert res.returncode == 0, res.stderr[:4000]
