@@ -102,6 +102,25 @@ __device__ __forceinline__ V3 axpy_m(double a, V3 x, V3 y) {
     return y;
 }
 
+// a x on the components x can have (M), zeros elsewhere
+template <int M>
+__device__ __forceinline__ V3 scale_m(double a, V3 x) {
+    return v3(bit(M, 0) ? a * x.x : 0.0, bit(M, 1) ? a * x.y : 0.0, bit(M, 2) ? a * x.z : 0.0);
+}
+
+// u + (w + p x q) with q's components in QM (and w's no others): the small terms
+// first, so that u is rounded once.  A step adds a hundredth of u or less, and what
+// is rounded off at the size of u, term by term, stays in the track.
+template <int QM>
+__device__ __forceinline__ V3 add_small(V3 u, V3 w, V3 p, V3 q) {
+    const V3 d = add_cross<QM>(w, p, q);
+    constexpr int M = QM | cross_bits(QM);
+    if constexpr (bit(M, 0)) u.x += d.x;
+    if constexpr (bit(M, 1)) u.y += d.y;
+    if constexpr (bit(M, 2)) u.z += d.z;
+    return u;
+}
+
 // beta^2, at most 0.9999 (pusher.py:74-96)
 __device__ __forceinline__ double clamped_beta2(V3 v) {
     const double bsq = dot_fma(v, v) * kInvC2;
@@ -224,23 +243,23 @@ __device__ __forceinline__ V3 boris_rel_u(V3 u, V3 E, V3 B, double dt, double qm
     const V3 t = (h * inv_gamma_u(um)) * B;
     const V3 s = (2.0 / (1.0 + dot_m<BM>(t, t))) * t;
     const V3 up = add_cross<BM>(um, um, t);
-    return axpy_m<EM>(h, E, add_cross<BM>(um, up, s));
+    return axpy_m<EM>(h, E, add_small<BM>(um, v3(0.0, 0.0, 0.0), up, s));
 }
 
 // Vay (2008); v_old = u / gamma(u).
 template <int EM, int BM>
 __device__ __forceinline__ V3 vay_u(V3 u, V3 v_old, V3 E, V3 B, double dt, double qm) {
     const double h = 0.5 * qm * dt;
-    // u' = u + (q/m) dt (E + v x B / 2)
+    // u' = u + (q/m) dt (E + v x B / 2), the increment added to u once
     const V3 tau = h * B;
-    const V3 up = add_cross<BM>(axpy_m<EM>(qm * dt, E, u), v_old, tau);
+    const V3 up = axpy_m<EM | cross_bits(BM)>(h, add_cross<BM>(scale_m<EM>(2.0, E), v_old, B), u);
     const double tau2 = dot_m<BM>(tau, tau);
     const double us = dot_m<BM>(up, tau) * kInvC;
     const double sigma = fma(dot_fma(up, up), kInvC2, 1.0) - tau2;
     const double ig = rsqrt(0.5 * (sigma + sqrt(fma(sigma, sigma, 4.0 * fma(us, us, tau2)))));
     const V3 t = ig * tau;
     const double s = 1.0 / fma(tau2, ig * ig, 1.0);
-    return s * add_cross<BM>(axpy_m<BM>(dot_m<BM>(up, t), t, up), up, t);
+    return s * add_small<BM>(up, scale_m<BM>(dot_m<BM>(up, t), t), up, t);
 }
 
 template <int ALG>
