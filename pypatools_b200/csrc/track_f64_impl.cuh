@@ -203,9 +203,10 @@ __device__ __forceinline__ V3 boris_v(V3 v, V3 E, V3 B, double dt, double qm) {
 template <int EM, int BM>
 __device__ __forceinline__ V3 vay_rel_v(V3 v, V3 E, V3 B, double dt, double qm) {
     const double qdt = qm * dt, h = 0.5 * qdt;
-    const V3 u = rsqrt(1.0 - clamped_beta2(v)) * v;
     const V3 tau = h * B;
-    const V3 up = axpy_m<EM>(qdt, E, u);
+    // gamma v + (q/m) E dt in one rounding: with u = gamma v rounded by itself, a kick
+    // far below u meets the same rounding at every step of a straight track
+    const V3 up = axpy(rsqrt(1.0 - clamped_beta2(v)), v, scale_m<EM>(qdt, E));
     const double tau2 = dot_m<BM>(tau, tau);
     const double q = dot_fma(up, tau) * kInvC;
     double gis = fma(-dot_fma(up, up), kInvC2, 1.0);

@@ -66,7 +66,7 @@ def _uniform(v):
     return Field.from_arrays({a: g for a in "xyz"}, comps) if comps else None
 
 
-@pytest.mark.parametrize("alg,field", [("vay", "ExEyBz"), ("vay", "full"), ("boris_rel", "B")])
+@pytest.mark.parametrize("alg,field", [("vay", "ExEyBz"), ("vay", "full"), ("boris_rel", "B"), ("vay_rel", "E")])
 def test_error_is_that_of_its_roundings(cuda, alg, field):
     import torch
     dev = torch.device("cuda", 0)
