@@ -1103,7 +1103,9 @@ static cudaError_t plan_resident(const int64_t n[3], int most, int padded_vector
 // Launch a resident kernel and read its report back (synchronises s).
 static int run_resident(const void* kernel, const ResidentPlan& plan, void** args, int64_t* iterations,
                         double* rel_residual, cudaStream_t s) {
-    PPT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+    // always the same limit: it belongs to the kernel, and another thread may be
+    // between its own setting and its launch
+    PPT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSharedLimit));
     PPT_CUDA_TRY(cudaMemsetAsync(plan.out, 0, sizeof(ResidentOut), s));
     if (plan.blocks > 1)
         PPT_CUDA_TRY(cudaMemsetAsync(plan.slots, 0, (size_t)plan.blocks * kSlotsPerBlock * sizeof(Slot), s));
