@@ -1100,6 +1100,11 @@ static cudaError_t plan_resident(const int64_t n[3], int most, int padded_vector
     return cudaSuccess;
 }
 
+// In place of a status: the device did not take the cooperative launch (its blocks
+// would not all be resident: SMs held by another partition or process), and
+// nothing of the solve has run.
+constexpr int kNotLaunched = 1;
+
 // Launch a resident kernel and read its report back (synchronises s).
 static int run_resident(const void* kernel, const ResidentPlan& plan, void** args, int64_t* iterations,
                         double* rel_residual, cudaStream_t s) {
@@ -1109,7 +1114,13 @@ static int run_resident(const void* kernel, const ResidentPlan& plan, void** arg
     PPT_CUDA_TRY(cudaMemsetAsync(plan.out, 0, sizeof(ResidentOut), s));
     if (plan.blocks > 1)
         PPT_CUDA_TRY(cudaMemsetAsync(plan.slots, 0, (size_t)plan.blocks * kSlotsPerBlock * sizeof(Slot), s));
-    PPT_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(plan.blocks), dim3(kResThreads), args, plan.smem, s));
+    const cudaError_t launched =
+        plan.polls > 0 ? cudaLaunchCooperativeKernel(kernel, dim3(plan.blocks), dim3(kResThreads), args, plan.smem, s)
+                       : cudaErrorCooperativeLaunchTooLarge;     // (a test's refusal)
+    if (launched != cudaSuccess) {
+        cudaGetLastError();          // an error of the context shows again in the launched form
+        return kNotLaunched;
+    }
     ResidentOut host;
     PPT_CUDA_TRY(cudaMemcpyAsync(&host, plan.out, sizeof(host), cudaMemcpyDeviceToHost, s));
     PPT_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1234,7 +1245,8 @@ static int solve_laplacian(const ppt_mesh_desc* mesh, const double* rhs, double*
                              : plan.per_thread == 4 ? (const void*)cg_resident<4>
                              : plan.per_thread == 8 ? (const void*)cg_resident<8>
                                                     : (const void*)cg_resident<12>;
-        return run_resident(kernel, plan, args, iterations, rel_residual, s);
+        rc = run_resident(kernel, plan, args, iterations, rel_residual, s);
+        if (rc != kNotLaunched) return rc;
     }
     cg_start<<<nb, kBlock, 0, s>>>(A, m, rhs, phi, r, p, part, part2);
     cg_scalars<<<1, kBlock, 0, s>>>(0, part, part2, nb, S, rel_tol, max_iter);
@@ -1324,7 +1336,8 @@ static int solve_coef(const ppt_mesh_desc* mesh, const double* coef, const doubl
                              : plan.per_thread == 2 ? (const void*)bi_resident<2>
                              : plan.per_thread == 4 ? (const void*)bi_resident<4>
                                                     : (const void*)bi_resident<8>;
-        return run_resident(kernel, plan, args, iterations, rel_residual, st);
+        rc = run_resident(kernel, plan, args, iterations, rel_residual, st);
+        if (rc != kNotLaunched) return rc;
     }
     bi_start<<<nb, kBlock, 0, st>>>(A, m, rhs, phi, r, rhat, p, v, part, part2);
     bi_scalars<<<1, kBlock, 0, st>>>(0, part, part2, nb, S, rel_tol, max_iter);
@@ -1351,8 +1364,9 @@ extern "C" int ppt_poisson_solve_coef(const ppt_mesh_desc* mesh, const double* c
     return solve_coef(mesh, coef, rhs, phi, scratch, rel_tol, max_iter, kSpinLimit, iterations, rel_residual, stream);
 }
 
-// The two solves (coef NULL: the first) with waits of at most `polls` polls:
-// how a test makes one run out.  Not part of the library's interface.
+// The two solves (coef NULL: the first) with waits of at most `polls` polls, how a
+// test makes one run out, or (0) with the cooperative launch refused.  Not part of
+// the library's interface.
 extern "C" int ppt_poisson_solve_polls(const ppt_mesh_desc* mesh, const double* coef, const double* rhs, double* phi,
                                        void* scratch, double rel_tol, int64_t max_iter, int polls, void* stream) {
     if (coef) return solve_coef(mesh, coef, rhs, phi, scratch, rel_tol, max_iter, polls, nullptr, nullptr, stream);
