@@ -782,10 +782,15 @@ __device__ __forceinline__ unsigned classify_row(const PoissonOp& A, const doubl
 // are read from coef at every use.
 struct Row {
     double w[7];
-    double inv;      // 1 / w[0]
-    double pad;      // an odd stride: the lanes' rows lie in all banks
+    double scale;    // what the preconditioner divides by, and its reciprocal
+    double inv;      // (nine doubles: an odd stride, so the lanes' rows lie in all banks)
 };
 constexpr int kFixedRows = 65;
+
+// The diagonal, or 1 where it cannot be divided by.
+__device__ __forceinline__ double row_scale(double diag) {
+    return diag != 0.0 && isfinite(1.0 / diag) ? diag : 1.0;
+}
 
 __device__ __forceinline__ double apply_row(const double* row, const double* x, int at, int sx, int sy) {
     const double w[6] = {row[1], row[2], row[3], row[4], row[5], row[6]};
@@ -796,7 +801,7 @@ constexpr double kRhoRounding = 1e-28;     // (1e-14)^2, of |rhat|^2 |r|^2
 
 // BiCGSTAB over per-cell rows with the diagonal as right preconditioner (the
 // residual and the stopping test stay those of the rows as they are):
-// A is applied to p^ = p / d and s^ = s / d, d the cell's diagonal.  A row next
+// A is applied to p^ = p / d and s^ = s / d, d the cell's diagonal (row_scale).  A row next
 // to a conductor surface a thousandth of a cell away has entries up to 1000
 // times the others'; without the division the iteration spends most of its
 // steps on them, and its rhat.r can vanish to rounding before it converges
@@ -836,6 +841,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     }
     for (int q = threadIdx.x; q < kFixedRows; q += kResThreads) {
         rows[q].w[0] = q == 64 ? 1.0 : A.diag;
+        rows[q].scale = rows[q].w[0];
         rows[q].inv = q == 64 ? 1.0 : inv_plain;
         for (int d = 0; d < 6; ++d) rows[q].w[1 + d] = q < 64 && (q & (1 << d)) ? A.off[d >> 1] : 0.0;
     }
@@ -845,7 +851,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     for (int h = threadIdx.x; h < P.halo; h += kResThreads) {
         const int pad = P.dst[h], i = pad / P.sx, j = (pad - i * P.sx) / P.sy, k = pad - i * P.sx - j * P.sy;
         const int64_t c = ((int64_t)(K.o[0] + i - 1) * B.n[1] + K.o[1] + j - 1) * B.n[2] + K.o[2] + k - 1;
-        halo_diag[h] = coef[7 * c];
+        halo_diag[h] = row_scale(coef[7 * c]);
         halo_inv[h] = halo_diag[h] == A.diag ? inv_plain : 1.0 / halo_diag[h];
         halo_v[h] = 0.0;
     }
@@ -874,7 +880,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 if (n < row_space) {
 #pragma unroll
                     for (int d = 0; d < 7; ++d) rows[n].w[d] = mine[d];
-                    rows[n].inv = mine[0] == A.diag ? inv_plain : 1.0 / mine[0];
+                    rows[n].scale = row_scale(mine[0]);
+                    rows[n].inv = rows[n].scale == A.diag ? inv_plain : 1.0 / rows[n].scale;
                     row[s] = n;
                 }
             }
@@ -909,10 +916,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
         inv = inv_plain;
         if (!(own[s] & kPlainWarp)) {
             if (row[s] >= 0) {
-                d = rows[row[s]].w[0];
+                d = rows[row[s]].scale;
                 inv = rows[row[s]].inv;
             } else {
-                d = coef[7 * (int64_t)(-1 - row[s])];
+                d = row_scale(coef[7 * (int64_t)(-1 - row[s])]);
                 inv = d == A.diag ? inv_plain : 1.0 / d;
             }
         }
