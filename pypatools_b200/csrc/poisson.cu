@@ -798,6 +798,7 @@ __device__ __forceinline__ double apply_row(const double* row, const double* x, 
 }
 
 constexpr double kRhoRounding = 1e-28;     // (1e-14)^2, of |rhat|^2 |r|^2
+constexpr double kSumRounding = 1e-10;     // of s.s: r.r = s.s - 2 omega t.s + omega^2 t.t to 1e-5 above it
 
 // BiCGSTAB over per-cell rows with the diagonal as right preconditioner (the
 // residual and the stopping test stay those of the rows as they are):
@@ -1014,11 +1015,19 @@ __global__ void __launch_bounds__(kResThreads, 1)
         }
         ++it;
         rr = fma(omega, fma(omega, sum[1], -2.0 * sum[0]), sum[4]);
-        if (rr < 0.0) rr = 0.0;                                  // s = omega t to rounding
         // (rhat.s vanishes but for rounding: without it rho would drift from rhat.r)
         const double rho_new = fma(-omega, sum[3], sum[2]);
         beta = omega != 0.0 ? (rho_new / rho) * (alpha / omega) : 0.0;
         rho = rho_new;
+        // near zero that is the rounding of its terms: before the solve ends on it, or the
+        // next step starts from it, r.r itself
+        if (rr <= tol2 || rr <= kSumRounding * sum[4] || it >= max_iter) {
+            double own_rr[1] = {0.0};
+#pragma unroll
+            for (int s = 0; s < S; ++s) own_rr[0] = fma(r[s], r[s], own_rr[0]);
+            if (!grid_sums(slots, out, polls, G, ++epoch, own_rr)) return;
+            rr = own_rr[0];
+        }
         done = rr <= tol2 || rr == 0.0 || it >= max_iter;
         // rhat.r is rounding alone (rhat lives on the cells with charge, r elsewhere by now)
         restart = omega == 0.0 || rho * rho <= kRhoRounding * rhat2 * rr;
