@@ -206,7 +206,24 @@ struct CoefOp {
     const double* coef;
 };
 
-enum { bRR = 0, bBB, bTOL2, bRHO, bALPHA, bOMEGA, bBETA, bDONE, bITERS, bNumScalars };
+enum { bRR = 0, bBB, bTOL2, bRHO, bRHAT2, bALPHA, bOMEGA, bBETA, bFRESH, bDONE, bITERS, bNumScalars };
+
+// Both forms of the iteration below (launched here, in one kernel further down)
+// have the diagonal as right preconditioner: A is applied to p^ = p / d and
+// s^ = s / d, and the residual and the stopping test stay those of the rows as they
+// are.  A row next to a conductor surface a thousandth of a cell away has entries up
+// to 1000 times the others'; without the division the iteration spends most of its
+// steps on them, and its rhat.r can vanish to rounding before it converges
+// (64 x 64 x 128 cells, pipe and aperture: 370-450 iterations to 1e-6, with it about
+// 140; 36 x 59 x 117 to 1e-8: stopped at residuals between 4e-9 and 0.16, with it 141
+// iterations).  Once rho = rhat.r is within the rounding of its sum, the iteration
+// starts again from r as its rhat.
+constexpr double kRhoRounding = 1e-28;     // (1e-14)^2, of |rhat|^2 |r|^2
+
+// The diagonal, or 1 where it cannot be divided by.
+__device__ __forceinline__ double row_scale(double diag) {
+    return diag != 0.0 && isfinite(1.0 / diag) ? diag : 1.0;
+}
 
 __device__ __forceinline__ double apply_coef(const CoefOp& A, const double* __restrict__ x, int64_t c) {
     const int64_t nz = A.n[2], sy = nz, sx = A.n[1] * nz;
@@ -244,13 +261,19 @@ __global__ void __launch_bounds__(kBlock) bi_start(const __grid_constant__ CoefO
     block_partial(bb, part2);
 }
 
-// p = r + beta (p - omega v)
-__global__ void __launch_bounds__(kBlock) bi_direction(int64_t m, const double* __restrict__ r, double* __restrict__ p,
-                                                       const double* __restrict__ v, const double* __restrict__ S) {
+// p^ = (r + beta (p - omega v)) / d, p holding p^; fresh: rhat = r, p^ = r / d
+__global__ void __launch_bounds__(kBlock) bi_direction(const __grid_constant__ CoefOp A, int64_t m,
+                                                       const double* __restrict__ r, double* __restrict__ rhat,
+                                                       double* __restrict__ p, const double* __restrict__ v,
+                                                       const double* __restrict__ S) {
     if (S[bDONE] != 0.0) return;
     const double beta = S[bBETA], omega = S[bOMEGA];
+    const bool fresh = S[bFRESH] != 0.0;
     const int64_t c = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (c < m) p[c] = r[c] + beta * (p[c] - omega * v[c]);
+    if (c >= m) return;
+    const double d = row_scale(A.coef[7 * c]), rc = r[c];
+    if (fresh) rhat[c] = rc;
+    p[c] = (fresh ? rc : rc + beta * (d * p[c] - omega * v[c])) / d;
 }
 
 // y = A z; partial sums of a.y (and of y.y when part2 is set)
@@ -274,16 +297,20 @@ __global__ void __launch_bounds__(kBlock) bi_apply(const __grid_constant__ CoefO
     }
 }
 
-// s = r - alpha v
-__global__ void __launch_bounds__(kBlock) bi_half(int64_t m, const double* __restrict__ r, const double* __restrict__ v,
-                                                  double* __restrict__ sv, const double* __restrict__ S) {
+// s = r - alpha v in r's place, s^ = s / d
+__global__ void __launch_bounds__(kBlock) bi_half(const __grid_constant__ CoefOp A, int64_t m, double* __restrict__ r,
+                                                  const double* __restrict__ v, double* __restrict__ sv,
+                                                  const double* __restrict__ S) {
     if (S[bDONE] != 0.0) return;
     const double alpha = S[bALPHA];
     const int64_t c = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (c < m) sv[c] = r[c] - alpha * v[c];
+    if (c >= m) return;
+    const double sc = r[c] - alpha * v[c];
+    r[c] = sc;
+    sv[c] = sc / row_scale(A.coef[7 * c]);
 }
 
-// x += alpha p + omega s, r = s - omega t; partial sums of rhat.r and r.r
+// x += alpha p^ + omega s^, r = s - omega t; partial sums of rhat.r and r.r
 __global__ void __launch_bounds__(kBlock) bi_update(int64_t m, double* __restrict__ x, double* __restrict__ r,
                                                     const double* __restrict__ rhat, const double* __restrict__ p,
                                                     const double* __restrict__ sv, const double* __restrict__ t,
@@ -295,7 +322,7 @@ __global__ void __launch_bounds__(kBlock) bi_update(int64_t m, double* __restric
     double d1 = 0.0, d2 = 0.0;
     if (c < m) {
         x[c] += alpha * p[c] + omega * sv[c];
-        const double rc = sv[c] - omega * t[c];
+        const double rc = r[c] - omega * t[c];
         r[c] = rc;
         d1 = rhat[c] * rc;
         d2 = rc * rc;
@@ -306,7 +333,7 @@ __global__ void __launch_bounds__(kBlock) bi_update(int64_t m, double* __restric
 }
 
 // One block.  mode 0: start; 1: alpha = rho / rhat.v; 2: omega = t.s / t.t;
-// 3: rho', beta, residual and the stopping test.
+// 3: rho', beta, residual and the stopping test, or a fresh start from r.
 __global__ void __launch_bounds__(kBlock) bi_scalars(int mode, const double* __restrict__ part,
                                                      const double* __restrict__ part2, int nb, double* S,
                                                      double rel_tol, int64_t max_iter) {
@@ -320,24 +347,31 @@ __global__ void __launch_bounds__(kBlock) bi_scalars(int mode, const double* __r
         S[bBB] = b;
         S[bTOL2] = rel_tol * rel_tol * b;
         S[bRHO] = a;          // rhat = r
+        S[bRHAT2] = a;
         S[bALPHA] = 1.0;
         S[bOMEGA] = 1.0;
-        S[bBETA] = 0.0;       // first direction p = r
+        S[bBETA] = 0.0;
+        S[bFRESH] = 1.0;      // first direction p = r
         S[bITERS] = 0.0;
         S[bDONE] = (a <= S[bTOL2] || a == 0.0 || max_iter <= 0) ? 1.0 : 0.0;
     } else if (mode == 1) {
-        S[bALPHA] = a != 0.0 ? S[bRHO] / a : 0.0;
-        if (a == 0.0) S[bDONE] = 1.0;                       // breakdown
+        S[bALPHA] = a != 0.0 ? S[bRHO] / a : 0.0;           // (0: the half step alone, then a fresh start)
     } else if (mode == 2) {
         S[bOMEGA] = b > 0.0 ? a / b : 0.0;                  // a = t.s, b = t.t
     } else {
         S[bITERS] += 1.0;
         S[bRR] = b;
         const double rho = a;
-        S[bBETA] = (S[bRHO] != 0.0 && S[bOMEGA] != 0.0) ? (rho / S[bRHO]) * (S[bALPHA] / S[bOMEGA]) : 0.0;
-        S[bRHO] = rho;
-        if (b <= S[bTOL2] || b == 0.0 || S[bITERS] >= (double)max_iter || rho == 0.0 || S[bOMEGA] == 0.0)
-            S[bDONE] = 1.0;
+        if (S[bOMEGA] == 0.0 || S[bALPHA] == 0.0 || rho * rho <= kRhoRounding * S[bRHAT2] * b) {
+            S[bRHO] = b;
+            S[bRHAT2] = b;
+            S[bFRESH] = 1.0;
+        } else {
+            S[bBETA] = (rho / S[bRHO]) * (S[bALPHA] / S[bOMEGA]);
+            S[bRHO] = rho;
+            S[bFRESH] = 0.0;
+        }
+        if (b <= S[bTOL2] || b == 0.0 || S[bITERS] >= (double)max_iter) S[bDONE] = 1.0;
     }
 }
 
@@ -787,33 +821,18 @@ struct Row {
 };
 constexpr int kFixedRows = 65;
 
-// The diagonal, or 1 where it cannot be divided by.
-__device__ __forceinline__ double row_scale(double diag) {
-    return diag != 0.0 && isfinite(1.0 / diag) ? diag : 1.0;
-}
-
 __device__ __forceinline__ double apply_row(const double* row, const double* x, int at, int sx, int sy) {
     const double w[6] = {row[1], row[2], row[3], row[4], row[5], row[6]};
     return apply_padded(row[0], w, x, at, sx, sy);
 }
 
-constexpr double kRhoRounding = 1e-28;     // (1e-14)^2, of |rhat|^2 |r|^2
 constexpr double kSumRounding = 1e-10;     // of s.s: r.r = s.s - 2 omega t.s + omega^2 t.t to 1e-5 above it
 
-// BiCGSTAB over per-cell rows with the diagonal as right preconditioner (the
-// residual and the stopping test stay those of the rows as they are):
-// A is applied to p^ = p / d and s^ = s / d, d the cell's diagonal (row_scale).  A row next
-// to a conductor surface a thousandth of a cell away has entries up to 1000
-// times the others'; without the division the iteration spends most of its
-// steps on them, and its rhat.r can vanish to rounding before it converges
-// (64 x 64 x 128 cells, pipe and aperture: 370-450 iterations to 1e-6, now about
-// 140; 36 x 59 x 117 to 1e-8: stopped at residuals between 4e-9 and 0.16, now 141
-// iterations).  p^ and s^ in padded bricks, x and rhat in shared memory, r (then
-// s), t, v and x in registers; p = d p^; of the padding cells r, v and d in lists.
-// rho = rhat.r and r.r come from the sums taken with t: r = s - omega t.  Once rho
-// is within the rounding of its sum, the iteration starts again from r as its
-// rhat; the launched form goes on, and stops unconverged where rho vanishes.  A warp
-// whose 32 cells all have the plain row takes its constants; another reads rows.
+// BiCGSTAB over per-cell rows (preconditioned and restarted as the launched form).
+// p^ and s^ in padded bricks, x and rhat in shared memory, r (then s), t, v and x in
+// registers; p = d p^; of the padding cells r, v and d in lists.  rho = rhat.r and
+// r.r come from the sums taken with t: r = s - omega t.  A warp whose 32 cells all
+// have the plain row takes its constants; another reads rows.
 template <int S>
 __global__ void __launch_bounds__(kResThreads, 1)
     bi_resident(const __grid_constant__ PoissonOp A, const __grid_constant__ Bricks B,
@@ -1359,11 +1378,11 @@ static int solve_coef(const ppt_mesh_desc* mesh, const double* coef, const doubl
     bi_scalars<<<1, kBlock, 0, st>>>(0, part, part2, nb, S, rel_tol, max_iter);
     PPT_CUDA_TRY(cudaGetLastError());
     rc = run_iterations(st, S, bDONE, bNumScalars, max_iter, host, [&](cudaStream_t ss) {
-        bi_direction<<<nb, kBlock, 0, ss>>>(m, r, p, v, S);
+        bi_direction<<<nb, kBlock, 0, ss>>>(A, m, r, rhat, p, v, S);
         bi_apply<<<nb, kBlock, 0, ss>>>(A, m, p, v, rhat, part, nullptr, S);
         bi_scalars<<<1, kBlock, 0, ss>>>(1, part, nullptr, nb, S, rel_tol, max_iter);
-        bi_half<<<nb, kBlock, 0, ss>>>(m, r, v, sv, S);
-        bi_apply<<<nb, kBlock, 0, ss>>>(A, m, sv, t, sv, part, part2, S);
+        bi_half<<<nb, kBlock, 0, ss>>>(A, m, r, v, sv, S);
+        bi_apply<<<nb, kBlock, 0, ss>>>(A, m, sv, t, r, part, part2, S);
         bi_scalars<<<1, kBlock, 0, ss>>>(2, part, part2, nb, S, rel_tol, max_iter);
         bi_update<<<nb, kBlock, 0, ss>>>(m, phi, r, rhat, p, sv, t, part, part2, S);
         bi_scalars<<<1, kBlock, 0, ss>>>(3, part, part2, nb, S, rel_tol, max_iter);
