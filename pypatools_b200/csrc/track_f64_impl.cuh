@@ -130,7 +130,8 @@ __device__ __forceinline__ double clamped_beta2(V3 v) {
 __device__ __forceinline__ V3 clamp_speed(V3 v) {
     constexpr double top = 0.9999 * kClight;
     const double v2 = dot_fma(v, v);
-    if (v2 >= top * top) v = v * (top * rsqrt(v2));
+    // (also where v2 is NaN: every component is then, whatever the record layout leaves out)
+    if (!(v2 < top * top)) v = v * (top * rsqrt(v2));
     return v;
 }
 
