@@ -11,6 +11,7 @@ from pathlib import Path
 LIB_PATH = Path(os.environ.get("PPT_LIBRARY", Path(__file__).resolve().parent / "lib" / "libppt.so"))
 
 PPT_OK = 0
+PPT_ERR_OOM = -2
 ERRORS = {-1: "PPT_ERR_ARG", -2: "PPT_ERR_OOM", -3: "PPT_ERR_CUDA", -4: "PPT_ERR_UNSUPPORTED",
           -5: "PPT_ERR_TIMEOUT", -6: "PPT_ERR_DEVICE"}
 
