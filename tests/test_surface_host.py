@@ -24,22 +24,25 @@ class _FakeLib:
         return b"fake"
 
 
-def _surface(monkeypatch, rc):
+@pytest.fixture
+def surface(monkeypatch):
     import torch
-    lib = _FakeLib(rc)
+    lib = _FakeLib(0)
     monkeypatch.setattr(electrodes._lib, "load", lambda: lib)
     monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
-    return ElectrodeSurface([[0.0, 0.0, 0.0], [1.0, 0.0, 0.0], [0.0, 1.0, 0.0]], [[0, 1, 2]])
+    s = ElectrodeSurface([[0.0, 0.0, 0.0], [1.0, 0.0, 0.0], [0.0, 1.0, 0.0]], [[0, 1, 2]])
+    yield s, lib
+    s._handles.clear()          # nothing of the stand-in's for the library to destroy
 
 
-def test_a_segment_grid_without_memory_leaves_the_surface_usable(monkeypatch):
-    s = _surface(monkeypatch, _lib.PPT_ERR_OOM)
+def test_a_segment_grid_without_memory_leaves_the_surface_usable(surface):
+    s, lib = surface
+    lib.refine = _lib.PPT_ERR_OOM
     assert s.handle("cuda:0", segments=True) == 1234
-    s._handles.clear()
 
 
-def test_another_error_of_it_is_raised(monkeypatch):
-    s = _surface(monkeypatch, -3)
+def test_another_error_of_it_is_raised(surface):
+    s, lib = surface
+    lib.refine = -3
     with pytest.raises(_lib.PptError):
         s.handle("cuda:0", segments=True)
-    s._handles.clear()
