@@ -650,10 +650,13 @@ class PusherGPU:
         df = self._device_fields(efield, bfield)
         tr = DeviceTracker(self.algorithm, self.q_over_m, df, m, 1, dt, 1, self.precision, record=False,
                            stagger=False, device=self.device, dt_rows=dt_rows)
-        # one copy each way
-        d_rv = self._upload(np.stack([r, v]), df.device)
+        # one copy each way, on the caller's stream: the staging ring may be full of
+        # another thread's track, which its rows are still waiting for
+        rv = torch.empty((2, m, 3), dtype=torch.float64, pin_memory=True)
+        rv[0], rv[1] = torch.from_numpy(r), torch.from_numpy(v)
         with torch.cuda.device(df.device):
             stream = torch.cuda.current_stream()
+            d_rv = rv.to(df.device, non_blocking=True)
             tr.load(d_rv[0], d_rv[1], stream)
             tr.advance(1, stream)
             tr.store(d_rv[0], d_rv[1], stream)
