@@ -26,6 +26,7 @@ All work runs in libppt.so kernels; there is no CPU fallback.
 """
 import math
 import mmap
+import threading
 import warnings
 
 import numpy as np
@@ -477,11 +478,11 @@ class HostStager:
     first touch would otherwise be slower than the link."""
 
     _by_device = {}
+    _by_device_lock = threading.Lock()
 
     def __init__(self, device, chunk=2 << 20, slots=96, threads=None):
         import ctypes
         import os
-        import threading
         torch = _torch()
         self.torch = torch
         self.device = device
@@ -500,10 +501,11 @@ class HostStager:
     def for_device(cls, device):
         import torch
         key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-        st = cls._by_device.get(key)
-        if st is None:
-            st = cls._by_device[key] = cls(torch.device("cuda", key))
-        return st
+        with cls._by_device_lock:               # one ring and one pool of threads per device
+            st = cls._by_device.get(key)
+            if st is None:
+                st = cls._by_device[key] = cls(torch.device("cuda", key))
+            return st
 
     def copy(self, src, dst, after=None):
         """Queue the copy of the contiguous device tensor ``src`` into the

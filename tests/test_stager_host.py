@@ -124,3 +124,23 @@ def test_no_data_race(tmp_path):
     for _ in range(3):
         res = subprocess.run([str(exe), "several_callers"], capture_output=True, text=True, timeout=300)
         assert res.returncode == 0, res.stderr[:4000]
+
+
+def test_a_device_has_one_stager(monkeypatch):
+    import threading
+    import time
+    from pypatools_b200.pusher import HostStager
+    made = []
+
+    def init(self, device):
+        made.append(self)
+        time.sleep(0.05)
+
+    monkeypatch.setattr(HostStager, "__init__", init)
+    monkeypatch.setattr(HostStager, "_by_device", {})
+    threads = [threading.Thread(target=HostStager.for_device, args=("cuda:0",)) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(made) == 1
