@@ -453,6 +453,8 @@ int ppt_stager_download(ppt_stager* s, void* dst, const void* src, int64_t bytes
  * calling thread's own downloads since its last finish. */
 int ppt_stager_finish(ppt_stager* s);
 
+/* Waits for what is queued.  A handle may be destroyed again (no later stager
+ * gets the same one); any other call with it is PPT_ERR_ARG. */
 int ppt_stager_destroy(ppt_stager* s);
 
 const char* ppt_last_error(void);

@@ -359,6 +359,25 @@ static void settle(ppt_stager* S, uint64_t before) {
     });
 }
 
+// A caller's handle is a number that no later stager gets, looked up here: a
+// handle that has been destroyed is an error (or nothing left to destroy), also for
+// an owner that does not know of it.
+struct StagerTable {
+    std::mutex m;
+    std::map<uintptr_t, ppt_stager*> live;
+    uintptr_t last = 0;
+};
+static StagerTable& stagers() {
+    static StagerTable* t = new StagerTable;      // outlives the threads of the process's end
+    return *t;
+}
+static ppt_stager* live_stager(ppt_stager* handle) {
+    StagerTable& t = stagers();
+    std::lock_guard<std::mutex> lock(t.m);
+    const auto at = t.live.find(reinterpret_cast<uintptr_t>(handle));
+    return at == t.live.end() ? nullptr : at->second;
+}
+
 // The stager's device is current while one of its calls runs.
 struct OnDevice {
     int prev = 0;
@@ -372,12 +391,7 @@ struct OnDevice {
     }
 };
 
-}  // namespace ppt
-
-using namespace ppt;
-
-extern "C" int ppt_stager_destroy(ppt_stager* S) {
-    if (!S) return PPT_OK;
+static void destroy_stager(ppt_stager* S) {
     // the waiter first: it hands its last arrivals to the pool
     if (!S->threads.empty() && (int)S->threads.size() > S->pool) {
         {
@@ -399,6 +413,23 @@ extern "C" int ppt_stager_destroy(ppt_stager* S) {
         if (S->pinned) cudaFreeHost(S->pinned);
     }
     delete S;
+}
+
+}  // namespace ppt
+
+using namespace ppt;
+
+extern "C" int ppt_stager_destroy(ppt_stager* handle) {
+    ppt_stager* S = nullptr;
+    {
+        StagerTable& t = stagers();
+        std::lock_guard<std::mutex> lock(t.m);
+        const auto at = t.live.find(reinterpret_cast<uintptr_t>(handle));
+        if (at == t.live.end()) return PPT_OK;
+        S = at->second;
+        t.live.erase(at);
+    }
+    destroy_stager(S);
     return PPT_OK;
 }
 
@@ -422,7 +453,7 @@ extern "C" int ppt_stager_create(int64_t slot_bytes, int n_slots, int n_threads,
             e = cudaEventCreateWithFlags(&S->slots[k].ev, cudaEventDisableTiming);
         }
         if (e != cudaSuccess) {
-            ppt_stager_destroy(S);
+            destroy_stager(S);
             return e == cudaErrorMemoryAllocation ? fail(PPT_ERR_OOM, "pinned staging buffers") : cuda_fail(e, "stager");
         }
         S->pool = n_threads;
@@ -430,16 +461,20 @@ extern "C" int ppt_stager_create(int64_t slot_bytes, int n_slots, int n_threads,
         S->threads.reserve((size_t)n_threads + 1);
         for (int t = 0; t < n_threads; ++t) S->threads.emplace_back(stager_worker, S, t);
         S->threads.emplace_back(stager_waiter, S);
+        StagerTable& t = stagers();
+        std::lock_guard<std::mutex> lock(t.m);
+        t.live.emplace(++t.last, S);
+        *out = reinterpret_cast<ppt_stager*>(t.last);
     } catch (const std::exception& ex) {
-        if (S) ppt_stager_destroy(S);
+        if (S) destroy_stager(S);
         return fail(PPT_ERR_OOM, std::string("stager: ") + ex.what());
     }
-    *out = S;
     return PPT_OK;
 }
 
-extern "C" int ppt_stager_upload(ppt_stager* S, void* dst, const void* src, int64_t bytes, void* stream) {
-    if (!S || bytes < 0 || (bytes > 0 && (!dst || !src))) return fail(PPT_ERR_ARG, "stager, dst and src must not be NULL");
+extern "C" int ppt_stager_upload(ppt_stager* handle, void* dst, const void* src, int64_t bytes, void* stream) {
+    ppt_stager* S = live_stager(handle);
+    if (!S || bytes < 0 || (bytes > 0 && (!dst || !src))) return fail(PPT_ERR_ARG, "not a stager, or dst or src NULL");
     if (bytes == 0) return PPT_OK;
     try {
         std::lock_guard<std::mutex> ring(S->ring);
@@ -461,8 +496,9 @@ extern "C" int ppt_stager_upload(ppt_stager* S, void* dst, const void* src, int6
     }
 }
 
-extern "C" int ppt_stager_download(ppt_stager* S, void* dst, const void* src, int64_t bytes, void* after) {
-    if (!S || bytes < 0 || (bytes > 0 && (!dst || !src))) return fail(PPT_ERR_ARG, "stager, dst and src must not be NULL");
+extern "C" int ppt_stager_download(ppt_stager* handle, void* dst, const void* src, int64_t bytes, void* after) {
+    ppt_stager* S = live_stager(handle);
+    if (!S || bytes < 0 || (bytes > 0 && (!dst || !src))) return fail(PPT_ERR_ARG, "not a stager, or dst or src NULL");
     try {
         std::lock_guard<std::mutex> ring(S->ring);
         OnDevice on(S->device);
@@ -476,8 +512,9 @@ extern "C" int ppt_stager_download(ppt_stager* S, void* dst, const void* src, in
     }
 }
 
-extern "C" int ppt_stager_finish(ppt_stager* S) {
-    if (!S) return fail(PPT_ERR_ARG, "stager is NULL");
+extern "C" int ppt_stager_finish(ppt_stager* handle) {
+    ppt_stager* S = live_stager(handle);
+    if (!S) return fail(PPT_ERR_ARG, "not a stager");
     try {
         std::unique_lock<std::mutex> lock(S->m);
         const uint64_t upto = S->queued;

@@ -28,6 +28,7 @@ import math
 import mmap
 import threading
 import warnings
+import weakref
 
 import numpy as np
 
@@ -456,7 +457,6 @@ def host_array(shape, dtype=np.float64):
     by their zeroing (50 GB/s), and into a recycled mapping by the copy
     alone.  The mapping returns to the pool when the array and every view of
     it are gone."""
-    import weakref
     nbytes = int(np.prod(shape)) * np.dtype(dtype).itemsize
     if nbytes < (4 << 20) or not hasattr(mmap, "MADV_HUGEPAGE"):
         return np.empty(shape, dtype)
@@ -496,6 +496,13 @@ class HostStager:
         with torch.cuda.device(device):
             _lib.check(self.lib.ppt_stager_create(int(chunk), int(slots), int(threads), self.stream.cuda_stream, handle))
         self.handle = handle.value
+        # its pinned memory and threads go with it (with what its last copies use; not at
+        # the process's end, which takes them anyway)
+        weakref.finalize(self, self._destroy, self.lib, self.handle, self.stream, self._copies).atexit = False
+
+    @staticmethod
+    def _destroy(lib, handle, stream, copies):
+        lib.ppt_stager_destroy(handle)
 
     @classmethod
     def for_device(cls, device):
@@ -544,7 +551,7 @@ class HostStager:
             landed = {id(c) for c in self._copies if c[2]}
         rc = self.lib.ppt_stager_finish(self.handle)
         with self._copies_lock:
-            self._copies = [c for c in self._copies if id(c) not in landed]
+            self._copies[:] = [c for c in self._copies if id(c) not in landed]
         _lib.check(rc)
 
 

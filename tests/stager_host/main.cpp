@@ -92,6 +92,20 @@ static void error_of_its_caller() {
     expect(ppt_stager_finish(ring.s) == PPT_OK, "once");
 }
 
+// A handle outlives its stager: destroying it again is nothing, using it an error,
+// and a later stager does not get it.
+static void destroyed_twice() {
+    FakeStream copy;
+    ppt_stager *first = nullptr, *second = nullptr;
+    char a[8] = {}, b[8] = {};
+    expect(ppt_stager_create(4096, 2, 1, &copy, &first) == PPT_OK, "create");
+    expect(ppt_stager_download(first, a, b, 8, nullptr) == PPT_OK, "a download that nothing waits for");
+    expect(ppt_stager_destroy(first) == PPT_OK && ppt_stager_destroy(first) == PPT_OK, "destroy twice");
+    expect(ppt_stager_create(4096, 2, 1, &copy, &second) == PPT_OK && second != first, "another one");
+    expect(ppt_stager_destroy(first) == PPT_OK && ppt_stager_finish(first) == PPT_ERR_ARG, "the old handle");
+    expect(ppt_stager_finish(second) == PPT_OK && ppt_stager_destroy(second) == PPT_OK, "the new one");
+}
+
 // Uploads and downloads from several threads: every byte (and, built with
 // -fsanitize=thread, no data race).
 static void several_callers() {
@@ -122,6 +136,7 @@ int main(int argc, char** argv) {
     if (which == "refused_download") refused_download();
     else if (which == "refused_upload") refused_upload();
     else if (which == "error_of_its_caller") error_of_its_caller();
+    else if (which == "destroyed_twice") destroyed_twice();
     else if (which == "several_callers") several_callers();
     else return 2;
     return 0;

@@ -31,7 +31,8 @@ def cases(tmp_path_factory):
     return _compile(tmp_path_factory.mktemp("stager"))
 
 
-@pytest.mark.parametrize("case", ["refused_download", "refused_upload", "error_of_its_caller", "several_callers"])
+@pytest.mark.parametrize("case", ["refused_download", "refused_upload", "error_of_its_caller", "destroyed_twice",
+                                  "several_callers"])
 def test_stager(cases, case):
     res = subprocess.run([str(cases), case], capture_output=True, text=True, timeout=120)
     assert res.returncode == 0, res.stderr
@@ -144,3 +145,36 @@ def test_a_device_has_one_stager(monkeypatch):
     for t in threads:
         t.join()
     assert len(made) == 1
+
+
+def test_a_dropped_stager_is_destroyed(monkeypatch):
+    import contextlib
+    import torch
+    from pypatools_b200 import pusher
+
+    class Lib(_FakeLib):
+        destroyed = []
+
+        def ppt_stager_create(self, chunk, slots, threads, stream, out):
+            out.value = 77
+            return 0
+
+        def ppt_stager_destroy(self, handle):
+            self.destroyed.append(handle)
+            return 0
+
+    class Stream:
+        cuda_stream = 5
+
+        def __init__(self, device):
+            pass
+
+    lib = Lib()
+    monkeypatch.setattr(pusher._lib, "load", lambda: lib)
+    monkeypatch.setattr(pusher, "_torch", lambda: torch)
+    monkeypatch.setattr(torch.cuda, "Stream", Stream)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    st = pusher.HostStager(torch.device("cuda", 0))
+    assert st.handle == 77 and not lib.destroyed
+    del st
+    assert lib.destroyed == [77]
