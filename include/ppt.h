@@ -267,8 +267,8 @@ int ppt_surface_destroy(ppt_surface* surface);
 
 /* Add a finer grid for the segment tests (ppt_track with a surface,
  * ppt_surface_segments_hit) and what tells a track how far from the surface it
- * is: the same hits, sooner.  Optional, once per surface,
- * before it is used by other threads; synchronises. */
+ * is: the same hits, sooner.  Optional, once per surface (again: nothing), while
+ * other threads may use it; synchronises. */
 int ppt_surface_refine(ppt_surface* surface);
 
 /* device bytes held, and the cell grid's dimensions */

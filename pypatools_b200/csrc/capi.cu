@@ -82,7 +82,7 @@ extern "C" int ppt_track(ppt_state* st, const ppt_fields* fields, const ppt_trac
         P.counters = a->counters;
         if (a->surface) {
             if (!a->active) return fail(PPT_ERR_ARG, "a surface needs the active array");
-            P.surf = a->surface->dev;
+            P.surf = a->surface->view();
             P.active = a->active;
         }
         if (a->dt_rows) {
@@ -107,7 +107,7 @@ extern "C" int ppt_track(ppt_state* st, const ppt_fields* fields, const ppt_trac
     if (rc) return rc;
     if (a->surface) {
         CollDev C;
-        C.surf = a->surface->dev;
+        C.surf = a->surface->view();
         C.active = a->active;
         return launch_track_mixed_coll(P, C, rf, s);
     }

@@ -285,6 +285,7 @@ extern "C" int ppt_surface_refine(ppt_surface* s) {
             return e == cudaErrorMemoryAllocation ? fail(PPT_ERR_OOM, "cudaMalloc of the segment grid failed")
                                                   : cuda_fail(e, "segment grid upload");
         }
+        std::lock_guard<std::mutex> lock(s->m);
         s->dev.clearance = reinterpret_cast<const uint8_t*>(base + b_start + b_list);
         if (f > 1) {
             D.clearance = s->dev.clearance;
@@ -320,7 +321,7 @@ extern "C" int ppt_surface_axis_rays(const ppt_surface* s, int64_t n, const doub
     if (n == 0) return PPT_OK;
     if (!points || !min_dist || !hits) return fail(PPT_ERR_ARG, "points, min_dist and hits must not be NULL");
     const int block = 128;
-    axis_rays_kernel<<<grid_for(n * 6, block), block, 0, static_cast<cudaStream_t>(stream)>>>(s->dev, n, points,
+    axis_rays_kernel<<<grid_for(n * 6, block), block, 0, static_cast<cudaStream_t>(stream)>>>(s->view(), n, points,
                                                                                               min_dist, hits);
     PPT_CUDA_TRY(cudaGetLastError());
     return PPT_OK;
@@ -344,6 +345,7 @@ extern "C" int ppt_surface_destroy(ppt_surface* s) {
 
 extern "C" int ppt_surface_info(const ppt_surface* s, int64_t* bytes, int32_t dims[3]) {
     if (!s) return fail(PPT_ERR_ARG, "surface is NULL");
+    std::lock_guard<std::mutex> lock(s->m);
     if (bytes) *bytes = (int64_t)s->bytes;
     if (dims)
         for (int a = 0; a < 3; ++a) dims[a] = s->dev.dims[a];
@@ -357,7 +359,7 @@ extern "C" int ppt_surface_segments_hit(const ppt_surface* s, int64_t n, const d
     if (n == 0) return PPT_OK;
     if (!p0 || !p1 || !hit) return fail(PPT_ERR_ARG, "p0, p1 and hit must not be NULL");
     const int block = 128;
-    segments_hit_kernel<<<grid_for(n, block), block, 0, static_cast<cudaStream_t>(stream)>>>(s->dev, n, p0, p1,
+    segments_hit_kernel<<<grid_for(n, block), block, 0, static_cast<cudaStream_t>(stream)>>>(s->view(), n, p0, p1,
                                                                                              hit);
     PPT_CUDA_TRY(cudaGetLastError());
     return PPT_OK;

@@ -305,5 +305,10 @@ struct ppt_surface {
     size_t bytes;
     std::vector<int32_t> start;  // the cells' list offsets
     std::vector<double> boxes;   // the triangles' bounding boxes (lo x y z, hi x y z)
-    std::mutex refining;
+    std::mutex refining;         // one ppt_surface_refine at a time
+    mutable std::mutex m;        // dev and bytes, which it changes while other threads use the surface
+    ppt::SurfaceDev view() const {
+        std::lock_guard<std::mutex> lock(m);
+        return dev;
+    }
 };
