@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(kBlock) bi_scalars(int mode, const double* __r
 // registers: the vectors of up to twelve cells per thread stay resident, and
 // latency is covered by cells instead of warps.
 // B200, us per iteration, launched form -> this one: CG on 16^3 / 52 x 52 x 54 /
-// 64 x 64 x 128 cells 12.5 / 15.2 / 19.4 -> 4.3 / 5.6 / 8.4; BiCGSTAB 20.8 / 28.5 /
-// 39.5 -> 10.6 / 14.5 / 26.6, with a third of the iterations (bi_resident).
+// 64 x 64 x 128 cells 12.5 / 15.2 / 19.4 -> 4.7 / 5.7 / 8.7; BiCGSTAB 20.8 / 28.5 /
+// 39.5 -> 11.3 / 14.8 / 27.9 (the launched form's before it had the preconditioner).
 // ---------------------------------------------------------------------------
 constexpr int kResThreads = 512;
 constexpr int kResWarps = kResThreads / 32;
@@ -416,7 +416,7 @@ struct alignas(16) Slot {
 
 // The slots of two waits in turn: every block's partial sums, sum by sum, then
 // the grid's: slots[(e & 1) * kResMaxSums * (blocks + 1) + ...].
-constexpr int kSlotsPerBlock = 4 * kResMaxSums;   // two waits, and as much again: at least two blocks
+constexpr int kSlotsPerBlock = 4 * kResMaxSums;   // two waits of blocks + 1 slots, for two blocks or more
 
 // What a solve reports: written by block 0 at its end (`finished` stays 0 when
 // it left before), and `late` by every block that gave up a wait.
@@ -478,8 +478,8 @@ __device__ __forceinline__ double warp_sums(const double (&a)[W], int lane, int 
 // each as one 16-byte word with the step's number.  With every block reading
 // all partial sums instead, a step among 148 blocks takes 4.1 us for one value,
 // 6.3 for two and 7.2 for five, since their polls of the same lines hold up one
-// another and the stores they wait for; so it takes 3.1 and 3.2 us for one and
-// for four.
+// another and the stores they wait for; so it took 3.1 and 3.2 us for one and
+// for four without lane 0's fence, which adds 0.1 to 0.4 us to an iteration.
 template <int N>
 __device__ __forceinline__ bool grid_sums(Slot* slots, ResidentOut* out, int polls, GridSums& G, unsigned long long e,
                                           double (&a)[N]) {
@@ -648,7 +648,9 @@ __device__ __forceinline__ void update_halo(const Padded& P, const double* pub, 
 
 // Of a thread's cell: its padded index (bits 0..15), kOwned, and kFace when
 // another block may read it.  The loops over a thread's cells have no branch on
-// kOwned around their arithmetic, so the cells' chains overlap.
+// kOwned around their arithmetic, so the cells' chains overlap.  (A thread without a
+// cell reads the brick's first one, perhaps while its owner writes it: what it makes
+// of it goes nowhere.)
 constexpr unsigned kOwned = 1u << 16, kFace = 1u << 17;
 constexpr unsigned kPlainWarp = 1u << 18;     // bi_resident: its warp's cells all have the plain row
 
@@ -1069,7 +1071,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
 
 // The bricks of a resident solve, its cells per thread (0: the mesh does not
 // fit) and its shared memory.  One block on each SM at most, and one per 1024
-// cells: a wait costs less among few blocks.  Of the ways to cut the mesh: the
+// cells, rounded up to 256 (two from 1793 cells): a wait costs less among few blocks.  Of the ways to cut the mesh: the
 // one with the fewest cells and padding cells per brick.
 struct ResidentPlan {
     Bricks bricks;
@@ -1124,10 +1126,10 @@ static cudaError_t plan_resident(const int64_t n[3], int most, int padded_vector
             }
         }
     // The slots lie in a vector of the scratch that the resident form leaves free
-    // (1024 cells and more for each block's 256 bytes; none for a single block);
+    // (896 cells and more for each block's 320 bytes; none for a single block);
     // a caller's scratch is aligned for doubles, the slots need 16 bytes.  The
     // report goes where the launched form keeps its sums.
-    static_assert(kSlotsPerBlock * sizeof(Slot) + 8 <= 1024 * sizeof(double), "a block's slots fit its cells' scratch");
+    static_assert(kSlotsPerBlock * sizeof(Slot) + 8 <= 896 * sizeof(double), "a block's slots fit its cells' scratch");
     static_assert(sizeof(ResidentOut) <= 9 * sizeof(double), "the report fits the sums' scratch");
     plan->slots = reinterpret_cast<Slot*>((reinterpret_cast<uintptr_t>(spare) + 15) & ~(uintptr_t)15);
     plan->out = reinterpret_cast<ResidentOut*>(sums);
@@ -1165,10 +1167,10 @@ static int run_resident(const void* kernel, const ResidentPlan& plan, void** arg
     return PPT_OK;
 }
 
-// Iterations of a solve on a mesh too large for the resident kernels: kIterPerGraph of them captured once as a CUDA graph
-// on a private stream (the caller's may be the legacy default stream, which
-// cannot be captured) and replayed until the device-side stop flag is set;
-// one host check per replay.  The kernels and their order are those of plain
+// Iterations of a solve that the resident kernels do not take (a larger mesh, or a
+// refused launch): kIterPerGraph of them captured once as a CUDA graph on a private
+// stream (the caller's may be the legacy default stream, which cannot be captured)
+// and replayed until the device-side stop flag is set; one host check per replay.  The kernels and their order are those of plain
 // launches, so the results are the same bits, with a fraction of the launch
 // cost (a solve is thousands of short launches on L2-resident vectors).
 constexpr int kIterPerGraph = 16;

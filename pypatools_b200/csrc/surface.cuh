@@ -231,7 +231,7 @@ __device__ __forceinline__ int clear_steps(const ClearBox& b, V3 p, V3 d) {
     for (int a = 0; a < 3; ++a)
         if (u[a] != 0.0) k = fmin(k, u[a] > 0.0 ? (hi[a] - x[a]) / u[a] : (lo[a] - x[a]) / u[a]);
     k = k * (1.0 - 1e-9) - 1.0;
-    return k >= 1.0 ? (int)k : 0;      // (NaN: 0)
+    return k >= 1.0 ? (int)k : 0;      // (a point that is NaN has no clear box, whose infinities give 0)
 }
 
 // Ray p + t d (t >= 0) against one triangle: the hit's t, or -1.  The same
