@@ -13,7 +13,8 @@ return shapes and error messages:
     change_algorithm(name), ALGORITHMS, __repr__
 
 and adds keyword-only options: ``precision`` ('fp64' = the reference method
-in float64, the drop-in; 'mixed' = the mixed-precision form), ``device``,
+in float64, the drop-in; 'mixed' = the mixed-precision form, faster for the
+Boris family and 'vay', slower for 'vay_rel' and 'rk4_rel'), ``device``,
 ``snapshot`` ('host' numpy arrays like the reference, or 'device' torch
 tensors), ``steps_per_launch``, ``sort_every`` (cell re-sort interval; 'auto' = every 300
 steps for bunches of 65536 or more, none below) and,
@@ -662,7 +663,8 @@ class PusherGPU:
         # one copy each way, on the caller's stream: the staging ring may be full of
         # another thread's track, which its rows are still waiting for
         rv = torch.empty((2, m, 3), dtype=torch.float64, pin_memory=True)
-        rv[0], rv[1] = torch.from_numpy(r), torch.from_numpy(v)
+        for k, a in enumerate((r, v)):
+            rv[k] = torch.from_numpy(a if a.flags.writeable else a.copy())   # (torch warns of read-only arrays)
         with torch.cuda.device(df.device):
             stream = torch.cuda.current_stream()
             d_rv = rv.to(df.device, non_blocking=True)

@@ -30,3 +30,15 @@ def test_a_push_does_not_wait_for_queued_copies(cuda):
     np.testing.assert_array_equal(got[0], expect[0])
     np.testing.assert_array_equal(got[1], expect[1])
     assert (host == 1.0).all()
+
+
+def test_read_only_arrays_raise_no_warning(cuda):
+    import warnings
+    g = np.linspace(-1.0, 1.0, 4)
+    field = Field.from_arrays({a: g for a in "xyz"}, {"z": np.ones((4, 4, 4))})
+    r, v = np.zeros((3, 3)), np.full((3, 3), 1e5)
+    r.flags.writeable = v.flags.writeable = False
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        r1, v1 = PusherGPU(IonSpecies("proton"), "boris").push_batch(r, v, None, field, 1e-9)
+    assert np.isfinite(r1).all() and np.isfinite(v1).all()

@@ -124,6 +124,8 @@ def test_no_data_race(tmp_path):
     exe = _compile(tmp_path, "-fsanitize=thread")
     for _ in range(3):
         res = subprocess.run([str(exe), "several_callers"], capture_output=True, text=True, timeout=300)
+        if "unexpected memory mapping" in res.stderr:          # the system's address layout, at random
+            pytest.skip("no ThreadSanitizer here")
         assert res.returncode == 0, res.stderr[:4000]
 
 
